@@ -642,6 +642,7 @@ __device__ int uf_find(int* uf, int x) {
 }
 
 // Breadth-first levels (one CTA).  Slot space: every contact vertex has a slot.
+constexpr int kLevelWarps = 32, kLevelTable = 128;
 __global__ void k_levels(DContacts c, int* deg, int* uf, int* dist, int* seed, int* cobst, int* cdeg1, int* cmin,
                          int* elev, int* lcount, int cap_levels) {
   __shared__ int changed;
@@ -728,7 +729,6 @@ __global__ void k_levels(DContacts c, int* deg, int* uf, int* dist, int* seed, i
     ++d;
   } while (changed);
   if (tid == 0) maxlvl = 0;
-  for (int l = tid; l < cap_levels + 1; l += nth) lcount[l] = 0;
   __syncthreads();
   for (int e = tid; e < S; e += nth) elev[e] = min(dist[c.s_slota[e]], dist[c.s_slotb[e]]);
   // the reference opens one level per breadth-first frontier, including the
@@ -737,6 +737,71 @@ __global__ void k_levels(DContacts c, int* deg, int* uf, int* dist, int* seed, i
     if (dist[s] < INF) atomicMax(&maxlvl, dist[s]);
   __syncthreads();
   const int nl = min(maxlvl + 1, cap_levels);
+  // level_order: the contacts of each level in contact order.  A warp takes a
+  // run of consecutive contacts; with the runs' counts per level added up, it
+  // knows where its own go, and hands out places 32 contacts at a time (lanes
+  // of one level in lane order).  One thread that places them one after the
+  // other needs 60 ns each: 0.42 ms of this kernel's 0.51 ms at 7.3k contacts (now 0.09 ms).
+  const int lane = tid & 31, warp = tid >> 5;
+  auto place = [&](int e0, int e1, int* next) {
+    for (int e = e0 + lane; e - lane < e1; e += 32) {
+      const int l = e < e1 ? min(elev[e], nl - 1) : -1;
+      const unsigned int same = __match_any_sync(0xffffffffu, l);
+      int at = 0;
+      const int leader = __ffs(same) - 1;
+      if (lane == leader && l >= 0) {
+        at = next[l];
+        next[l] = at + __popc(same);
+      }
+      at = __shfl_sync(0xffffffffu, at, leader);
+      if (l >= 0) c.level_order[at + __popc(same & ((1u << lane) - 1u))] = e;
+      __syncwarp();
+    }
+  };
+  if (nl <= kLevelTable) {
+    __shared__ int table[kLevelWarps][kLevelTable];
+    const int per = (S + kLevelWarps - 1) / kLevelWarps;
+    const int e0 = min(S, warp * per), e1 = min(S, e0 + per);
+    for (int k = tid; k < kLevelWarps * kLevelTable; k += nth) (&table[0][0])[k] = 0;
+    __syncthreads();
+    for (int e = e0 + lane; e < e1; e += 32) atomicAdd(&table[warp][min(elev[e], nl - 1)], 1);
+    __syncthreads();
+    if (warp == 0) {
+      int acc = 0;  // contacts of the levels before the 32 of this round
+      for (int l0 = 0; l0 < nl; l0 += 32) {
+        const int l = l0 + lane;
+        int n = 0;
+        if (l < nl)
+          for (int w = 0; w < kLevelWarps; ++w) {
+            const int t = table[w][l];
+            table[w][l] = n;
+            n += t;
+          }
+        int incl = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += t;
+        }
+        const int start = acc + incl - n;
+        if (l < nl) {
+          c.level_ptr[l] = start;
+          for (int w = 0; w < kLevelWarps; ++w) table[w][l] += start;
+        }
+        acc += __shfl_sync(0xffffffffu, incl, 31);
+      }
+      if (lane == 0) {
+        c.level_ptr[nl] = acc;
+        *c.n_levels = nl;
+      }
+    }
+    __syncthreads();
+    place(e0, e1, table[warp]);
+    return;
+  }
+  // more levels than the table holds (long chains of contacts): one warp
+  for (int l = tid; l < nl; l += nth) lcount[l] = 0;
+  __syncthreads();
   for (int e = tid; e < S; e += nth) atomicAdd(lcount + min(elev[e], nl - 1), 1);
   __syncthreads();
   if (tid == 0) {
@@ -748,9 +813,9 @@ __global__ void k_levels(DContacts c, int* deg, int* uf, int* dist, int* seed, i
     }
     c.level_ptr[nl] = acc;
     *c.n_levels = nl;
-    // stable fill in contact order
-    for (int e = 0; e < S; ++e) c.level_order[lcount[min(elev[e], nl - 1)]++] = e;
   }
+  __syncthreads();
+  if (warp == 0) place(0, S, lcount);
 }
 
 void ws_alloc(SelfWS& w, int nv, int nt, int hit_cap, int slot_cap) {
@@ -990,7 +1055,7 @@ int self_detect_step(pdf_handle* h) {
 
 void self_levels_step(pdf_handle* h) {
   SelfWS& w = *(SelfWS*)h->d.self_ws;
-  k_levels<<<1, 1024, 0, h->stream>>>(h->d.c, w.deg, w.uf, w.dist, w.seed, w.cobst, w.cdeg1, w.cmin, w.elev,
+  k_levels<<<1, 32 * kLevelWarps, 0, h->stream>>>(h->d.c, w.deg, w.uf, w.dist, w.seed, w.cobst, w.cdeg1, w.cmin, w.elev,
                                       w.lcount, h->cap_self);
 }
 
