@@ -572,6 +572,7 @@ void build_sweep_plan(const Factor& f, int chunk, int cut_level, SweepPlan& plan
         for (int64_t t = f.sn_ftile0[s]; t < f.sn_ftile0[s + 1]; ++t) {
           const int tl = (int)(t - f.sn_ftile0[s]);
           const int w = std::min(f.sn_ns[s], kTile * tl + kTile);
+          if (w > kBlockSpanF && kTile * tl < f.sn_ns[s]) fb.split = 1;
           for (int a = 0; a < w; a += kBlockSpanF)
             plan.fitem.push_back(block_item(f.ftile_off[t], (int)f.sn_roff[s], 0, f.sn_c0[s] - fb.c0, f.sn_ns[s],
                                             f.sn_nr[s], tl, a, std::min(w, a + kBlockSpanF)));

@@ -127,6 +127,7 @@ struct SweepBlock {
   int item0;     // first item of the block in the item array
   int ext0;      // its ext rows are Factor::rows[ext0, ext0 + next) (R of the root)
   int next;
+  int split;     // a forward tile is split into spans: y of the columns has to start at zero
   int lev[kMaxBlockLevels + 1];  // item offsets (from item0) per level, in sweep order
 };
 // One work item of a tile of a supernode inside a block: forward, rows

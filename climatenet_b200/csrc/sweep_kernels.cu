@@ -386,6 +386,9 @@ __global__ void __launch_bounds__(kBlockMaxThreads, 1) k_block_forward(DPlan P, 
     stage_items(sm.items, P.fitem + B.item0, nitems);
     for (int e = threadIdx.x; e < B.next; e += blockDim.x) sv[nc + e] = sv[ld + nc + e] = sv[2 * ld + nc + e] = T(0);
     if (threadIdx.x <= nlev) s_lev[threadIdx.x] = B.lev[threadIdx.x];
+    if (B.split)  // spans add into y, which holds the last solve's
+      for (int k = threadIdx.x; k < nc; k += blockDim.x)
+        y[c0b + k] = y[(int64_t)n + c0b + k] = y[2 * (int64_t)n + c0b + k] = T(0);
     cp_async_wait_all();
     __syncthreads();
     if (warp == 0) {
@@ -454,7 +457,7 @@ __global__ void __launch_bounds__(kBlockMaxThreads, 1) k_block_forward(DPlan P, 
               y[o] = ax;
               y[o + n] = ay;
               y[o + 2 * (int64_t)n] = az;
-            } else {  // one span of a split tile (y starts at zero)
+            } else {  // one span of a split tile (y was cleared)
               atomicAdd(y + o, ax);
               atomicAdd(y + o + n, ay);
               atomicAdd(y + o + 2 * (int64_t)n, az);
