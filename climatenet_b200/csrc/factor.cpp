@@ -35,7 +35,7 @@ inline double dotn(const double* a, const double* b, int n) {
 
 // Nested dissection.  The separators of the top `merge` levels of the
 // dissection tree are not given their own supernodes: they are deferred and
-// ordered last, as one dense root supernode (top()), which removes merge - 1
+// ordered after the rest of the component, as one dense root supernode (top()), which removes merge - 1
 // levels from the elimination tree the device sweeps walk level by level.
 struct NDBuilder {
   const Model& m;
@@ -105,6 +105,32 @@ struct NDBuilder {
   }
 };
 
+// Connected components of the matrix graph: vertices ascending, components
+// by their lowest vertex.
+std::vector<std::vector<int>> components(const Model& m) {
+  std::vector<int> comp(m.N, -1), stack;
+  std::vector<std::vector<int>> out;
+  for (int r = 0; r < m.N; ++r) {
+    if (comp[r] >= 0) continue;
+    const int c = (int)out.size();
+    out.emplace_back();
+    comp[r] = c;
+    stack.push_back(r);
+    while (!stack.empty()) {
+      const int v = stack.back();
+      stack.pop_back();
+      for (int k = m.ata_ptr[v]; k < m.ata_ptr[v + 1]; ++k) {
+        const int j = m.ata_col[k];
+        if (comp[j] >= 0) continue;
+        comp[j] = c;
+        stack.push_back(j);
+      }
+    }
+  }
+  for (int v = 0; v < m.N; ++v) out[comp[v]].push_back(v);
+  return out;
+}
+
 // Top dissection levels merged into the root supernode (PDF_ND_MERGE
 // overrides it for tuning experiments).
 int nd_merge_levels() {
@@ -155,10 +181,14 @@ bool factorize(const Model& m, double dt, int leaf_size, Factor& f, std::string&
   // ---- ordering and supernode partition -------------------------------
   NDBuilder nd(m, std::max(8, leaf_size), nd_merge_levels());
   {
-    std::vector<int> ids(N);
-    std::iota(ids.begin(), ids.end(), 0);
-    nd.run(ids);
-    nd.top();
+    // each connected component of the matrix graph (a layer, a cloth of a
+    // batch) on its own: dissected together, components that overlap in space
+    // share supernodes, whose dense blocks hold a zero for every pair of rows of
+    // different components (three 128 x 128 layers: 16.5 M stored entries against 6.1 M)
+    for (std::vector<int>& ids : components(m)) {
+      nd.run(ids);
+      nd.top();
+    }
   }
   f.perm = nd.order;
   f.iperm.assign(N, 0);
