@@ -119,6 +119,7 @@ void build_schedule(pdf_handle* h, int chunk, int cut_level, int upper_mode = 0,
   P.rows_loc = upload(hp.rows_loc);
   P.bidx = upload(hp.bidx.empty() ? std::vector<int>(kSlabMax, 0) : hp.bidx);
   P.child = upload(hp.child.empty() ? std::vector<int>(2, 0) : hp.child);
+  P.chunk = chunk;
   P.max_cols = hp.max_block_cols;
   P.max_ext = hp.max_block_ext;
   P.max_items = hp.max_block_items;

@@ -51,6 +51,8 @@ struct DPlan {
   int max_items;        // most tiles of a block in one sweep
   int smem_f, smem_b;   // dynamic shared memory of the forward / backward block kernels
   int grid_bf, grid_bb, grid_uf, grid_ub;
+  int grid_lf, grid_lb;  // most CTAs of a level launch
+  int chunk;             // widest upper item (columns / rows)
   // launch shape of the block kernels (kBlockShapes): warps per CTA, CTAs
   // per SM it was sized for, and bulk-copy stages per warp (forward, backward)
   int block_shape, block_warps, block_ctas, ring_f, ring_b;

@@ -29,7 +29,7 @@
 //     is counted (each item counts itself without reading the counter back).
 //     Partial sums land in y / b_R with atomics.
 //  3. the same supernodes backward, top-down, in 32-column tiles x row
-//     chunks (k_upper_level_backward per level, or k_upper_backward with an
+//     chunks (k_upper_level per level, or k_upper_backward with an
 //     item waiting until its parent is complete); sums land in x.
 //  4. k_block_backward — the blocks top-down: their y slice and the final x
 //     of their ext rows are loaded into shared memory, the factor and, per
@@ -850,124 +850,167 @@ __global__ void __launch_bounds__(kSweepThreads) k_upper_backward(DPlan P, const
 // ---------------------------------------------- upper items, level by level
 
 // One elimination-tree level of upper items per launch, [lo, hi), spread
-// over all warps (grid-stride); the launches follow one another in sweep
-// order, so an item needs no dependency wait and signals nothing.  Launched
-// as programmatic dependents: an item's factor tile and row indices are
-// loaded before the wait for the previous launch, its vector after it.
-// Resident CTAs per SM the level kernels are compiled for: 3 in FP32 (its
-// 32-element tiles leave room; measured 4 % faster solves), 2 in FP64 (at 3
-// the FP64 kernels spill and the solve is 26 % slower).
-template <typename T>
-struct LevelOccupancy {
-  static constexpr int kCtas = sizeof(T) == 4 ? 3 : 2;
+// over all warps; the launches follow one another in sweep order, so an item
+// needs no dependency wait and signals nothing.  Launched as programmatic
+// dependents: an item's factor tile and row indices are read before the wait
+// for the previous launch, its vectors after it.
+//
+// A level's time is the boundary (some 3.6 us) and its bytes; they overlap as
+// far as the next level's tiles can already be on their way.  So the CTAs are
+// small (4 warps) and hold their tiles in shared memory instead of registers:
+// a warp copies its items by bulk copies into slots of its own (16 KB of them),
+// and 3 CTAs fit an SM whichever launches they belong to, with 192 KB (28 MB on
+// the GPU) in flight; as the CTAs of a level finish, those of the next one take
+// their place and fill their slots.  500 x 500 cloth, 8 levels a sweep: 64 us
+// forward and 69 us backward in FP64 (tiles in registers, 16 warps an SM: 71
+// and 70), the solve 0.248 ms (0.275); 97 x 97: 0.049 ms (0.053).
+// The grid is what is resident; more CTAs with one or two items a warp were
+// slower (0.256 and 0.276 ms), and so were fewer, which let the next level's
+// in from the start (2 and 1 per SM: 0.277 and 0.317 ms).
+constexpr int kLevelWarps = 4;
+template <typename T, int kSegs>
+struct LevelSlots {
+  static constexpr int kElems = 32 * 32 * kSegs;
+  static constexpr int kCount = (16384 / (int)sizeof(T)) / kElems > 1 ? (16384 / (int)sizeof(T)) / kElems : 1;
+  // per warp: its slots, 32 staged vector entries (4 values each), its barriers
+  static constexpr size_t kBytes = (kCount * kElems + 32 * 4) * sizeof(T) + kCount * sizeof(uint64_t);
 };
 
-template <typename T>
-__global__ void __launch_bounds__(kSweepThreads, LevelOccupancy<T>::kCtas) k_upper_level_forward(DPlan P, int lo, int hi,
-                                                                       const T* __restrict__ W, T* b, T* y, int n) {
-  const int lane = threadIdx.x & 31;
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-  griddep_launch_dependents();
-  bool waited = false;
-#pragma unroll 1
-  for (int t = lo + gw; t < hi; t += nwarps) {
-    const UpperItem tk = P.fup[t];
-    const int mrows = min(kTile, tk.ns + tk.nr - tk.tile * kTile);
-    const T* wbase = W + tk.off + lane;
-    const int row = tk.tile * kTile + lane;
-    const int64_t r = (row >= tk.ns && row < tk.ns + tk.nr) ? P.rows[tk.roff + row - tk.ns] : -1;
-    const T* bx = b + tk.c0;
-    const T* by = bx + n;
-    const T* bz = by + n;
-    T ax = 0, ay = 0, az = 0;
-    for (int j0 = tk.a0; j0 < tk.a1; j0 += 32) {
-      T w[32];
-      load_tile(w, wbase + (int64_t)j0 * mrows, min(32, tk.a1 - j0), mrows, lane < mrows);
-      if (!waited) {  // the factor is in flight; b comes from the previous launches
-        griddep_wait();
-        waited = true;
-      }
-      const int jl = j0 + lane;
-      T vx = 0, vy = 0, vz = 0;
-      if (jl < tk.a1) {
-        vx = ldcg(bx + jl);
-        vy = ldcg(by + jl);
-        vz = ldcg(bz + jl);
-      }
-#pragma unroll
-      for (int u = 0; u < 32; ++u) {
-        ax += w[u] * __shfl_sync(0xffffffffu, vx, u);
-        ay += w[u] * __shfl_sync(0xffffffffu, vy, u);
-        az += w[u] * __shfl_sync(0xffffffffu, vz, u);
-      }
-    }
-    if (row < tk.ns) {
-      const int64_t o = (int64_t)tk.c0 + row;
-      atomicAdd(y + o, ax);
-      atomicAdd(y + o + n, ay);
-      atomicAdd(y + o + 2 * (int64_t)n, az);
-    } else if (r >= 0) {
-      atomicAdd(b + r, -ax);
-      atomicAdd(b + r + n, -ay);
-      atomicAdd(b + r + 2 * (int64_t)n, -az);
-    }
-  }
-  // every thread waits before it exits, so that this launch completes only
-  // after the one before it (the next programmatic dependent relies on it)
-  if (!waited) griddep_wait();
+__device__ __forceinline__ void stage_vec(float* vs, float x, float y, float z) {
+  *reinterpret_cast<float4*>(vs) = make_float4(x, y, z, 0.f);
+}
+__device__ __forceinline__ void stage_vec(double* vs, double x, double y, double z) {
+  *reinterpret_cast<double2*>(vs) = make_double2(x, y);
+  vs[2] = z;
+}
+__device__ __forceinline__ void fma_vec(const float* vs, float w, float& ax, float& ay, float& az) {
+  const float4 v = *reinterpret_cast<const float4*>(vs);
+  ax += w * v.x;
+  ay += w * v.y;
+  az += w * v.z;
+}
+__device__ __forceinline__ void fma_vec(const double* vs, double w, double& ax, double& ay, double& az) {
+  const double2 v = *reinterpret_cast<const double2*>(vs);
+  ax += w * v.x;
+  ay += w * v.y;
+  az += w * vs[2];
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kSweepThreads, LevelOccupancy<T>::kCtas) k_upper_level_backward(DPlan P, int lo, int hi,
-                                                                        const T* __restrict__ W,
-                                                                        const T* __restrict__ y, T* x, int n) {
-  const int lane = threadIdx.x & 31;
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+template <typename T, bool kFwd, int kSegs>
+__global__ void __launch_bounds__(32 * kLevelWarps)
+    k_upper_level(DPlan P, int lo, int hi, const T* __restrict__ W, T* b, T* y, T* x, int n, SweepSync sy) {
+  constexpr int kSlotElems = LevelSlots<T, kSegs>::kElems, kLevelSlots = LevelSlots<T, kSegs>::kCount;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  T* ring = reinterpret_cast<T*>(smem_raw) + (size_t)warp * kLevelSlots * kSlotElems;
+  T* vs = reinterpret_cast<T*>(smem_raw) + (size_t)kLevelWarps * kLevelSlots * kSlotElems + warp * 32 * 4;
+  uint64_t* full = reinterpret_cast<uint64_t*>(reinterpret_cast<T*>(smem_raw) +
+                                               (size_t)kLevelWarps * (kLevelSlots * kSlotElems + 32 * 4)) +
+                   warp * kLevelSlots;
+  const int gw = blockIdx.x * kLevelWarps + warp, nwarps = gridDim.x * kLevelWarps;
   griddep_launch_dependents();
+  if (lane == 0) {
+    for (int k = 0; k < kLevelSlots; ++k) mbar_init(full + k, 1);
+    fence_mbar_init();
+  }
+  __syncwarp();
+  const UpperItem* items = (kFwd ? P.fup : P.bup) + lo;
+  const int count = hi - lo;
+  // lane 0 starts the copy of item t into a slot whose last tile is read
+  auto issue = [&](int t, int slot) {
+    if (t < count && lane == 0) {
+      const UpperItem& I = items[t];
+      const int j0 = kTile * I.tile;
+      const int width = kFwd ? min(kTile, I.ns + I.nr - j0) : min(kTile, I.ns - j0);
+      const uint32_t bytes = round16((uint32_t)(width * (I.a1 - I.a0)) * (uint32_t)sizeof(T));
+      fence_proxy_async();
+      mbar_expect_tx(full + slot, bytes);
+      bulk_g2s(ring + (size_t)slot * kSlotElems, W + I.off + (int64_t)width * I.a0, bytes, full + slot);
+    }
+  };
+#pragma unroll
+  for (int k = 0; k < kLevelSlots; ++k) issue(gw + k * nwarps, k);
   bool waited = false;
 #pragma unroll 1
-  for (int t = lo + gw; t < hi; t += nwarps) {
-    const UpperItem tk = P.bup[t];
-    const int mcols = min(kTile, tk.ns - tk.tile * kTile);
-    const T* wbase = W + tk.off + lane;
-    const int j0t = tk.tile * kTile;
-    const int col = j0t + lane;
-    const int nd = tk.ns - j0t;
-    T ax = 0, ay = 0, az = 0;
-    for (int i0 = tk.a0; i0 < tk.a1; i0 += 32) {
-      T w[32];
-      load_tile(w, wbase + (int64_t)i0 * mcols, min(32, tk.a1 - i0), mcols, lane < mcols);
-      const int il = i0 + lane;
-      const int64_t r = (il < tk.a1 && il >= nd) ? P.rows[tk.roff + il - nd] : 0;
-      if (!waited) {  // the factor and row indices are in flight; y and x come from the previous launches
-        griddep_wait();
-        waited = true;
-      }
-      T vx = 0, vy = 0, vz = 0;
-      if (il < tk.a1) {
-        if (il < nd) {
-          const int64_t o = (int64_t)tk.c0 + j0t + il;
-          vx = ldcg(y + o);
-          vy = ldcg(y + o + n);
-          vz = ldcg(y + o + 2 * (int64_t)n);
-        } else {
-          vx = -ldcg(x + r);
-          vy = -ldcg(x + r + n);
-          vz = -ldcg(x + r + 2 * (int64_t)n);
-        }
-      }
+  for (int t = gw, u = 0; t < count; t += nwarps, ++u) {
+    const UpperItem tk = items[t];
+    const int j0t = kTile * tk.tile, cnt = tk.a1 - tk.a0;
+    const int nd = tk.ns - j0t;  // backward: local rows of D^-1
+    const int m = min(kTile, kFwd ? nd + tk.nr : nd);
+    // forward: where the lane's row is in b; backward: where the rows are in x
+    int r[kSegs];
+    if (kFwd) {
+      r[0] = (lane >= nd && lane < m) ? P.rows[tk.roff + lane - nd] : -1;
+    } else {
 #pragma unroll
-      for (int u = 0; u < 32; ++u) {
-        ax += w[u] * __shfl_sync(0xffffffffu, vx, u);
-        ay += w[u] * __shfl_sync(0xffffffffu, vy, u);
-        az += w[u] * __shfl_sync(0xffffffffu, vz, u);
+      for (int g = 0; g < kSegs; ++g) {
+        const int il = tk.a0 + 32 * g + lane;
+        r[g] = (32 * g + lane < cnt && il >= nd) ? P.rows[tk.roff + il - nd] : -1;
       }
     }
-    if (col < tk.ns) {
-      const int64_t o = (int64_t)tk.c0 + col;
-      atomicAdd(x + o, ax);
-      atomicAdd(x + o + n, ay);
-      atomicAdd(x + o + 2 * (int64_t)n, az);
+    if (!waited) {  // b, y and x come from the previous launches
+      griddep_wait();
+      waited = true;
+    }
+    T v[kSegs][3];
+#pragma unroll
+    for (int g = 0; g < kSegs; ++g) {
+      const int l = 32 * g + lane;
+      v[g][0] = v[g][1] = v[g][2] = T(0);
+      if (l < cnt) {
+        const T* p = kFwd ? b + tk.c0 + tk.a0 + l : (r[g] >= 0 ? x + r[g] : y + tk.c0 + j0t + tk.a0 + l);
+        v[g][0] = ldcg(p);
+        v[g][1] = ldcg(p + n);
+        v[g][2] = ldcg(p + 2 * (int64_t)n);
+      }
+    }
+    const int slot = u % kLevelSlots;
+    if (!mbar_wait_warp(full + slot, (u / kLevelSlots) & 1, sy.max_spins)) {
+      if (lane == 0) atomicOr(sy.err, 1);
+      // no copy of this warp lands after the CTA exits
+      for (int k = 0; k < kLevelSlots; ++k)
+        if (t + k * nwarps < count)
+          mbar_wait_warp(full + (u + k) % kLevelSlots, ((u + k) / kLevelSlots) & 1, sy.max_spins);
+      break;
+    }
+    const T* w = ring + (size_t)slot * kSlotElems + min(lane, m - 1);
+    T ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0;
+#pragma unroll
+    for (int g = 0; g < kSegs; ++g) {
+      const int c = min(32, cnt - 32 * g);
+      if (c > 0) {
+        const T sg = !kFwd && r[g] >= 0 ? T(-1) : T(1);
+        stage_vec(vs + 4 * lane, sg * v[g][0], sg * v[g][1], sg * v[g][2]);
+        __syncwarp();
+        if (c == 32) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 2) {
+            fma_vec(vs + 4 * j, w[m * j], ax, ay, az);
+            fma_vec(vs + 4 * j + 4, w[m * j + m], bx, by, bz);
+          }
+        } else {
+#pragma unroll 8
+          for (int j = 0; j < c; ++j) fma_vec(vs + 4 * j, w[m * j], ax, ay, az);
+        }
+        w += 32 * m;
+        __syncwarp();
+      }
+    }
+    issue(t + kLevelSlots * nwarps, slot);  // the slot is read
+    ax += bx;
+    ay += by;
+    az += bz;
+    if (lane < m) {
+      T* out = kFwd ? y + tk.c0 + j0t + lane : x + tk.c0 + j0t + lane;
+      if (kFwd && r[0] >= 0) {
+        out = b + r[0];
+        ax = -ax;
+        ay = -ay;
+        az = -az;
+      }
+      atomicAdd(out, ax);
+      atomicAdd(out + n, ay);
+      atomicAdd(out + 2 * (int64_t)n, az);
     }
   }
   // every thread waits before it exits, so that this launch completes only
@@ -1053,6 +1096,18 @@ int resident_ctas(K kernel, size_t smem, int threads = kSweepThreads) {
   return per_sm * sms;
 }
 
+template <typename T>
+size_t level_smem_bytes(int chunk) {
+  return kLevelWarps * (chunk == 32   ? LevelSlots<T, 1>::kBytes
+                        : chunk == 64 ? LevelSlots<T, 2>::kBytes
+                                      : LevelSlots<T, 4>::kBytes);
+}
+// k_upper_level for items of up to chunk columns (rows)
+template <typename T, bool kFwd>
+auto level_kernel(int chunk) {
+  return chunk == 32 ? k_upper_level<T, kFwd, 1> : chunk == 64 ? k_upper_level<T, kFwd, 2> : k_upper_level<T, kFwd, 4>;
+}
+
 // The largest ring (kMinSlots .. kMaxSlots slots per CTA) with which `ctas`
 // CTAs of `warps` consumer warps and the producer warp of this block kernel
 // are resident per SM; 0 if none.
@@ -1088,10 +1143,10 @@ bool configure_solve(DPlan& P, int shape) {
   P.grid_bb = std::max(1, std::min(rb, std::max(1, P.nblk)));
   P.grid_uf = std::max(1, resident_ctas(k_upper_forward<T>, 0));
   P.grid_ub = std::max(1, resident_ctas(k_upper_backward<T>, 0));
-  // the level kernels use the same launch shape; make sure they can launch
-  resident_ctas(k_upper_level_forward<T>, 0);
-  resident_ctas(k_upper_level_backward<T>, 0);
-  return rf > 0 && rb > 0;
+  const size_t level = level_smem_bytes<T>(P.chunk);
+  P.grid_lf = resident_ctas(level_kernel<T, true>(P.chunk), level, 32 * kLevelWarps);
+  P.grid_lb = resident_ctas(level_kernel<T, false>(P.chunk), level, 32 * kLevelWarps);
+  return rf > 0 && rb > 0 && P.grid_lf > 0 && P.grid_lb > 0;
 }
 
 // Launch as a programmatic dependent of the previous kernel in the stream
@@ -1118,25 +1173,19 @@ void launch_solve_sweeps(cudaStream_t st, const DPlan& P, const T* Wf, const T* 
   // marks (optional): 4 events recorded between the five launches
   k_block_forward<T><<<P.grid_bf, 32 * (P.block_warps + 1), P.smem_f, st>>>(P, Wf, b, y, n, sy);
   if (marks) cudaEventRecord(marks[0], st);
+  auto level = [&](bool fwd, int lo, int hi) {
+    const int grid = std::max(1, std::min(fwd ? P.grid_lf : P.grid_lb, (hi - lo + kLevelWarps - 1) / kLevelWarps));
+    launch_dependent(fwd ? level_kernel<T, true>(P.chunk) : level_kernel<T, false>(P.chunk), grid, 32 * kLevelWarps,
+                     level_smem_bytes<T>(P.chunk), st, P, lo, hi, fwd ? Wf : Wb, b, y, x, n, sy);
+  };
   if (P.upper_mode == 1) {
-    const int wpc = kSweepThreads / 32;
-    for (int k = 0; k < P.n_flev; ++k) {
-      const int lo = P.flev[k], hi = P.flev[k + 1];
-      const int grid = std::max(1, std::min(P.grid_uf, (hi - lo + wpc - 1) / wpc));
-      launch_dependent(k_upper_level_forward<T>, grid, kSweepThreads, 0, st, P, lo, hi, Wf, b, y, n);
-    }
+    for (int k = 0; k < P.n_flev; ++k) level(true, P.flev[k], P.flev[k + 1]);
   } else {
     k_upper_forward<T><<<P.grid_uf, kSweepThreads, 0, st>>>(P, Wf, b, y, n, sy);
   }
   if (marks) cudaEventRecord(marks[1], st);
   if (P.upper_mode == 1) {
-    const int wpc = kSweepThreads / 32;
-    for (int k = 0; k < P.n_blev; ++k) {
-      const int lo = P.blev[k], hi = P.blev[k + 1];
-      const int grid = std::max(1, std::min(P.grid_ub, (hi - lo + wpc - 1) / wpc));
-      launch_dependent(k_upper_level_backward<T>, grid, kSweepThreads, 0, st, P, lo, hi, Wb,
-                       static_cast<const T*>(y), x, n);
-    }
+    for (int k = 0; k < P.n_blev; ++k) level(false, P.blev[k], P.blev[k + 1]);
   } else {
     k_upper_backward<T><<<P.grid_ub, kSweepThreads, 0, st>>>(P, Wb, y, x, n, sy);
   }
