@@ -169,6 +169,7 @@ void build_schedule(pdf_handle* h, int chunk, int cut_level, int upper_mode = 0,
 }
 
 void autotune_schedule(pdf_handle* h);
+bool build_dense(pdf_handle* h);
 
 // Warm-start feature / prediction buffers and the impulse memory.
 void ensure_mlp_buffers(pdf_handle* h) {
@@ -526,7 +527,7 @@ void create_impl(pdf_handle* h, const pdf_scene_desc* sc, const pdf_params* p) {
     }
   }
   CK(cudaDeviceSynchronize());
-  autotune_schedule(h);
+  if (!build_dense(h)) autotune_schedule(h);
   // the timing solves overwrote v and q^k: restore the initial state
   CK(cudaMemcpy(d.v, m.v0.data(), m.v0.size() * sizeof(double), cudaMemcpyHostToDevice));
   CK(cudaMemcpy(d.qk, m.q0.data(), m.q0.size() * sizeof(double), cudaMemcpyHostToDevice));
@@ -551,14 +552,24 @@ void launch_local(pdf_handle* h, T* b, int mode) {
                        std::max(h->prm.air_damping, 0.), d.c.slot_of, d.c.f, b, h->prm.time_step, mode);
 }
 
-// Global solve: one persistent forward and one backward sweep (which writes
+// The inverse in the precision of the solve (b only picks it).
+inline const double* dense_of(const DeviceBuffers& d, const double*) { return d.dense64; }
+inline const float* dense_of(const DeviceBuffers& d, const float*) { return d.dense32; }
+
+// Global solve: for small scenes one product with the inverse; else one persistent forward and one backward sweep (which writes
 // back v and q^k of the blocks' columns), then the write-back of the upper
 // columns (which also clears their x, y for the next solve).
 template <typename T>
 void launch_solve(pdf_handle* h, T* b, T* y, T* x, const T* Wf, const T* Wb, int mode) {
   DeviceBuffers& d = h->d;
-  launch_solve_sweeps<T>(h->stream, d.plan, Wf, Wb, b, y, x, h->dm.N, d.sync,
-                         WriteBack{d.v, d.qk, d.q, h->prm.time_step, mode});
+  const WriteBack wb{d.v, d.qk, d.q, h->prm.time_step, mode};
+  if (d.dense) {
+    const T* A = dense_of(d, b);
+    if (!launch_dense_solve<T>(h->stream, d.dense_rows, A, b, h->dm.N, d.dense_np, d.perm, wb, h->dm.trace))
+      throw CudaFail("the dense solve does not fit the device's shared memory");
+    return;
+  }
+  launch_solve_sweeps<T>(h->stream, d.plan, Wf, Wb, b, y, x, h->dm.N, d.sync, wb);
 }
 
 template <typename T>
@@ -566,6 +577,105 @@ void launch_solve_with(pdf_handle* h, const SweepSync& sy, T* b, T* y, T* x, con
   DeviceBuffers& d = h->d;
   launch_solve_sweeps<T>(h->stream, d.plan, Wf, Wb, b, y, x, h->dm.N, sy,
                          WriteBack{d.v, d.qk, d.q, h->prm.time_step, mode});
+}
+
+// Small scenes (kDenseBytes): the explicit inverse, its columns three at a time
+// by the FP64 sweeps (whatever the precision of the solve), one captured solve
+// replayed.  false where the scene is too large.
+bool build_dense(pdf_handle* h) {
+  DeviceBuffers& d = h->d;
+  const Factor& f = h->fac;
+  const int N = h->dm.N;
+  const size_t s = h->fp32 ? sizeof(float) : sizeof(double);
+  const int pad = 16 / (int)s;
+  std::vector<DenseRow> rows(N);
+  int64_t total = 0;
+  int widest = 0, np = 0;
+  for (size_t c = 0; c + 1 < f.comp_ptr.size(); ++c) {
+    const int c0 = f.comp_ptr[c], n = f.comp_ptr[c + 1] - c0, ld = (n + pad - 1) / pad * pad;
+    if ((uint64_t)n * ld > kDenseBytes / s) return false;
+    for (int r = 0; r < n; ++r) rows[c0 + r] = DenseRow{total + (int64_t)r * ld, c0, n, np - c0};
+    np += ld;
+    total += (int64_t)n * ld;
+    widest = std::max(widest, n);
+    if ((uint64_t)total > kDenseBytes / s) return false;
+  }
+  if (3 * (size_t)np * s > (size_t)kDenseSmem) return false;
+  d.dense_np = np;
+  cudaStream_t st = h->stream;
+  d.dense_rows = upload(rows);
+  if (h->fp32)
+    d.dense32 = dalloc<float>(total);
+  else
+    d.dense64 = dalloc<double>(total);
+  CK(cudaMemsetAsync(h->fp32 ? (void*)d.dense32 : (void*)d.dense64, 0, total * s, st));  // the rows' padding
+  // FP64 sweeps on scratch vectors (the handle's own where it solves in FP64)
+  const bool fp32 = h->fp32;
+  std::vector<void*> tmp;
+  auto scratch = [&](size_t n) {
+    double* p = dalloc<double>(n);
+    tmp.push_back(p);
+    return p;
+  };
+  double *Wf = d.Wf64, *Wb = d.Wb64, *b = d.b64, *y = d.y64, *x = d.x64;
+  double *v = nullptr, *qk = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  int* column = nullptr;
+  auto release = [&] {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (column) cudaFree(column);
+    for (void* p : tmp) cudaFree(p);
+    h->fp32 = fp32;
+  };
+  try {
+    h->fp32 = false;
+    // leaves and their parents as blocks, 32-column items, 2 CTAs of 8 warps
+    build_schedule(h, 32, 1, 1, 1);
+    if (fp32) {
+      tmp.push_back(Wf = upload(f.Wf));
+      tmp.push_back(Wb = upload(f.Wb));
+      b = scratch(3 * (size_t)N);
+      y = scratch(3 * (size_t)N);
+      x = scratch(3 * (size_t)N);
+    }
+    v = scratch(3 * (size_t)N);
+    qk = scratch(3 * (size_t)N);
+    column = dalloc<int>(1);
+    CK(cudaMemsetAsync(column, 0, sizeof(int), st));
+    SweepSync sy = d.sync;
+    sy.trace.stamps = nullptr;
+    launch_solve_prep<double>(st, N, x, y, sy);
+    cudaGraph_t g;
+    CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    launch_dense_unit(st, d.dense_rows, b, N, column);
+    launch_solve_sweeps<double>(st, d.plan, Wf, Wb, b, y, x, N, sy, WriteBack{v, qk, d.q, 0., 0});
+    if (fp32)
+      launch_dense_rows<float>(st, d.dense_rows, v, N, d.perm, d.dense32, column);
+    else
+      launch_dense_rows<double>(st, d.dense_rows, v, N, d.perm, d.dense64, column);
+    CK(cudaStreamEndCapture(st, &g));
+    const cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
+    cudaGraphDestroy(g);
+    CK(e);
+    for (int k = 0; k < widest; k += 3) CK(cudaGraphLaunch(exec, st));
+    CK(cudaStreamSynchronize(st));
+    int derr = 0;
+    CK(cudaMemcpy(&derr, d.sync.err, sizeof(int), cudaMemcpyDeviceToHost));
+    if (derr) throw CudaFail("a supernodal sweep gave up waiting while the inverse was built");
+  } catch (...) {
+    release();
+    throw;
+  }
+  release();
+  // the schedule the sweeps would take, should pdf_set_sweep_schedule ask for them
+  build_schedule(h, 32, 1, 1, 1);
+  if (fp32)
+    launch_solve_prep<float>(st, N, d.x32, d.y32, d.sync);
+  else
+    launch_solve_prep<double>(st, N, d.x64, d.y64, d.sync);
+  CK(cudaStreamSynchronize(st));
+  d.dense = true;
+  return true;
 }
 
 // Schedule autotuner: times the global solve of this scene's factor with
@@ -701,9 +811,10 @@ void launch_iteration(pdf_handle* h, T* b, T* y, T* x, const T* Wf, const T* Wb,
 }
 
 // Kernels of this library launched by one PD iteration (CUB's not counted):
-// [bending], vertex rhs, friction, [self friction], forward, backward, post, AC.
+// [bending], vertex rhs, friction, [self friction], forward, backward, post (small
+// scenes: one product), AC.
 int64_t launches_per_iteration(const pdf_handle* h) {
-  return 6 + (h->dm.B > 0 ? 1 : 0) + (h->prm.self_collision ? 1 : 0);
+  return (h->d.dense ? 4 : 6) + (h->dm.B > 0 ? 1 : 0) + (h->prm.self_collision ? 1 : 0);
 }
 
 // Per step outside the iterations: predictor, obstacle flags + clamp + materialise,
@@ -1034,7 +1145,7 @@ void free_handle(pdf_handle* h) {
                   d.c.s_ac, d.c.s_slota, d.c.s_slotb, d.c.s_remember, d.c.n_levels, d.c.level_ptr,
                   d.c.level_order, d.c.slot_of, d.c.n_slots, d.c.slot_vertex, d.c.f, d.c.cf[0], d.c.cf[1],
                   d.c.sf[0], d.c.sf[1], d.c.c_gap, d.c.c_active, h->mlp_w, h->mlp_X, h->mlp_Y, h->rprev,
-                  h->rprev_tag, h->log_X, h->log_T, h->log_n, d.iter, d.iter_total, d.blocks_done, d.stamps,
+                  h->rprev_tag, h->log_X, h->log_T, h->log_n, d.iter, d.iter_total, d.blocks_done, d.stamps, d.dense_rows, d.dense64, d.dense32,
                   d.c.ac_trace, h->gather_idx, h->gather_out, h->stage, h->bad_dev, d.ob_best};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -1606,7 +1717,13 @@ int pdf_time_solve_parts(pdf_handle* h, int32_t reps, double* part_ms) {
       CK(cudaMemcpyAsync(bcur, bsave, bbytes, cudaMemcpyDeviceToDevice, st));
       CK(cudaEventRecord(ev[0], st));
       WriteBack wb{d.v, d.qk, d.q, h->prm.time_step, h->fp32 ? 1 : 0};
-      if (h->fp32)
+      if (d.dense) {  // one launch: the first part
+        if (h->fp32)
+          launch_solve<float>(h, d.b32, d.y32, d.x32, d.Wf32, d.Wb32, 1);
+        else
+          launch_solve<double>(h, d.b64, d.y64, d.x64, d.Wf64, d.Wb64, 0);
+        for (int k = 1; k < 5; ++k) CK(cudaEventRecord(ev[k], st));
+      } else if (h->fp32)
         launch_solve_sweeps<float>(st, d.plan, d.Wf32, d.Wb32, d.b32, d.y32, d.x32, N, d.sync, wb, ev + 1);
       else
         launch_solve_sweeps<double>(st, d.plan, d.Wf64, d.Wb64, d.b64, d.y64, d.x64, N, d.sync, wb, ev + 1);
@@ -1640,6 +1757,7 @@ int pdf_set_sweep_schedule(pdf_handle* h, int32_t chunk, int32_t cut_level, int3
   return guarded(h, [&]() -> int {
     CK(cudaSetDevice(h->prm.device));
     CK(cudaStreamSynchronize(h->stream));
+    h->d.dense = false;
     build_schedule(h, chunk, cut_level, upper_mode, block_shape);
     const bool mode_ok = h->d.plan.upper_mode == upper_mode && h->d.plan.block_shape == block_shape;
     if (!mode_ok) build_schedule(h, chunk, cut_level, 0, 0);

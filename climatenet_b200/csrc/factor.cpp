@@ -186,9 +186,11 @@ bool factorize(const Model& m, double dt, int leaf_size, Factor& f, std::string&
     // share supernodes, whose dense blocks hold a zero for every pair of rows of
     // different components (three 128 x 128 layers: 16.5 M stored entries against 6.1 M)
     for (std::vector<int>& ids : components(m)) {
+      f.comp_ptr.push_back((int)nd.order.size());
       nd.run(ids);
       nd.top();
     }
+    f.comp_ptr.push_back((int)nd.order.size());
   }
   f.perm = nd.order;
   f.iperm.assign(N, 0);

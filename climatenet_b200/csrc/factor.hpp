@@ -61,6 +61,7 @@ struct Factor {
   std::vector<int64_t> sn_ftile0, sn_btile0;
   std::vector<int64_t> ftile_off, btile_off;  // per tile, +1 sentinel
   std::vector<double> Wf, Wb;
+  std::vector<int> comp_ptr;     // connected components: columns [comp_ptr[c], comp_ptr[c + 1])
   int n_levels = 0;
   int64_t nnz_w = 0;             // sum ns(ns+1)/2 + nr ns
   int64_t nnz_l_true = 0;        // structural nnz of L (diagonal included)

@@ -176,6 +176,30 @@ void launch_solve_sweeps(cudaStream_t st, const DPlan& P, const T* Wf, const T* 
 template <typename T>
 void launch_solve_prep(cudaStream_t st, int n, T* x, T* y, SweepSync sy);
 
+// Small scenes: the solve as one product with the explicit inverse
+// (dense_solve.cu).  The inverse is kept where it takes at most kDenseBytes and
+// b fits the kernel's shared memory (two CTAs an SM).  Below the limit the product
+// reads L2-resident rows and beats the sweeps' chain of launches (30 x 30 FP64:
+// 6.5 MB, 10 us against 33; at the limit, 64 x 64 FP32: 23 us against 47); above
+// it the inverse grows with N^2 where the factor grows with N log N, and leaves L2.
+// Its construction (a third of N solves) replaces the schedule autotuner there:
+// creating a 30 x 30 cloth takes as long as before, a 61 x 61 FP32 one 84 ms
+// instead of 53.
+constexpr size_t kDenseBytes = size_t(64) << 20;
+constexpr int kDenseSmem = 100 * 1024;
+struct DenseRow {
+  int64_t off;  // first entry of the row
+  int c0, n;    // its component: first column, columns
+  int shift;    // c0 + shift is where the component's entries start in a padded plane
+};
+template <typename T>
+bool launch_dense_solve(cudaStream_t st, const DenseRow* rows, const T* A, const T* b, int n, int np,
+                        const int* perm, WriteBack wb, DTrace trace);  // np: entries of a padded plane
+void launch_dense_unit(cudaStream_t st, const DenseRow* rows, double* b, int n, const int* column);
+template <typename T>
+void launch_dense_rows(cudaStream_t st, const DenseRow* rows, const double* v, int n, const int* perm, T* A,
+                       int* column);
+
 // detection (detect_kernels.cu, compiled without FMA contraction)
 __global__ void k_obstacle_flags(int N, const double* q, DObstacles obs, unsigned char* flags);
 __global__ void k_obstacle_materialize(int N, const double* q, DObstacles obs, const int* idx, const int* vmat,
