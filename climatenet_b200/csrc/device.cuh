@@ -24,6 +24,18 @@ __device__ __forceinline__ unsigned long long global_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
+// Programmatic dependent launch: a kernel launched with the programmatic
+// stream serialization attribute (launch_dependent) may start while the kernel
+// before it in the stream still runs; griddep_wait() returns once that kernel has
+// completed and its memory operations are visible.  Before it, such a kernel
+// reads only data that no kernel of its chain writes.  Every thread waits before
+// it exits, so that a launch completes only after its predecessor.
+// griddep_launch_dependents() lets the next such kernel start launching.
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void griddep_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // called by every thread; only thread 0 of block 0 writes
 __device__ __forceinline__ void trace_stamp(const DTrace& t, int row) {
   if (t.stamps && blockIdx.x == 0 && threadIdx.x == 0) {

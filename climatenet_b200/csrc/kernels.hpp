@@ -3,10 +3,29 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include <utility>
+
 #include "device.cuh"
 #include "factor.hpp"
 
 namespace pdfb {
+
+// Launch as a programmatic dependent of the previous kernel in the stream
+// (the kernel calls griddep_wait() before it reads what that kernel writes).
+template <typename... Params, typename... Args>
+void launch_dependent(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t st, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
 
 // Work queues (4 ints: forward / backward upper items, forward / backward
 // blocks), solve counter and cumulative completion counters.

@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "device.cuh"
+#include "kernels.hpp"
 #include "mlp.hpp"
 
 namespace pdfb {
@@ -201,172 +202,341 @@ __global__ void k_mlp_forward(const float* __restrict__ prm, const float* __rest
   }
 }
 
-// Gradient of the mean squared error over the samples idx[0..n) (or 0..n
-// when idx is null), accumulated into grad (kMlpParams) and loss.
-__global__ void k_mlp_grad(const float* __restrict__ prm, const float* __restrict__ X, const float* __restrict__ T,
-                           const int* __restrict__ idx, int n, float* __restrict__ grad, double* __restrict__ loss) {
-  extern __shared__ unsigned char smem[];
-  SmemWeights& w = *reinterpret_cast<SmemWeights*>(smem);
-  float* g = reinterpret_cast<float*>(smem + sizeof(SmemWeights));  // kMlpParams gradients
-  WarpBuf* bufs = reinterpret_cast<WarpBuf*>(smem + sizeof(SmemWeights) + sizeof(float) * ((kMlpParams + 63) / 64 * 64));
-  load_weights(w, prm);
-  for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x) g[i] = 0.f;
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
-  WarpBuf& b = bufs[warp];
-  const float inv_n = 1.f / (float)n;
-  double lsum = 0.;
-  for (int s0 = (blockIdx.x * nw + warp) * 16; s0 < n; s0 += gridDim.x * nw * 16) {
-    for (int i = lane; i < 16 * 16; i += 32) {
-      const int r = i / 16, c = i % 16;
-      float v = 0.f;
-      if (c < kIn && s0 + r < n) {
-        const int64_t sidx = idx ? idx[s0 + r] : (s0 + r);
-        v = X[sidx * kIn + c];
-      }
-      b.x[i] = v;
-    }
-    __syncwarp();
-    warp_forward(w, b);
-    // output gradient dL/dy = 2 (y - t) / n  (rows past n and cols >= 3 are zero)
-    for (int i = lane; i < 16 * 8; i += 32) {
-      const int r = i / 8, c = i % 8;
-      float d = 0.f;
-      if (c < kOut && s0 + r < n) {
-        const int64_t sidx = idx ? idx[s0 + r] : (s0 + r);
-        const float e = b.y[i] - T[sidx * kOut + c];
-        lsum += (double)e * e;
-        d = 2.f * e * inv_n;
-      }
-      b.y[i] = d;
-    }
-    __syncwarp();
-    // dW3 += dY^T h2: A(r, k) = dY(k, r) (16 x 16, rows >= 8 read as zero via padding), B = h2 (k x n)
-    for (int nt = 0; nt < kH / 8; ++nt) {
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
-      uint32_t a[4], bb[2];
-      // rows 8..15 of dY^T do not exist: use a zero-padded view by reading
-      // column r of dY only for r < 8
-      {
-        const int g2 = lane >> 2, t = lane & 3;
-        auto e = [&](int r, int k) { return r < 8 ? b.y[k * 8 + r] : 0.f; };
-        a[0] = pack_bf16(e(g2, 2 * t), e(g2, 2 * t + 1));
-        a[1] = pack_bf16(e(g2 + 8, 2 * t), e(g2 + 8, 2 * t + 1));
-        a[2] = pack_bf16(e(g2, 2 * t + 8), e(g2, 2 * t + 9));
-        a[3] = pack_bf16(e(g2 + 8, 2 * t + 8), e(g2 + 8, 2 * t + 9));
-      }
-      load_b(bb, b.h2, kH, 1, 0, nt * 8);
-      mma16816(c, a, bb);
-      const int g2 = lane >> 2, t = lane & 3;
-      // rows g2 (< 8) hold dW3[g2][n]; only rows < 3 are parameters
-      if (g2 < kOut) {
-        atomicAdd(&g[OW3 + g2 * kH + nt * 8 + 2 * t], c[0]);
-        atomicAdd(&g[OW3 + g2 * kH + nt * 8 + 2 * t + 1], c[1]);
-      }
-    }
-    for (int c = lane; c < kOut; c += 32) {
-      float s = 0.f;
-      for (int r = 0; r < 16; ++r) s += b.y[r * 8 + c];
-      atomicAdd(&g[OB3 + c], s);
-    }
-    // dH2 = dY W3 (16 x 64): A = dY (16 x 16, cols >= 8 zero), B(k, n) = w3[k][n]
-    for (int nt = 0; nt < kH / 8; ++nt) {
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
-      uint32_t a[4], bb[2];
-      {
-        const int g2 = lane >> 2, t = lane & 3;
-        auto ea = [&](int r, int k) { return k < 8 ? b.y[r * 8 + k] : 0.f; };
-        a[0] = pack_bf16(ea(g2, 2 * t), ea(g2, 2 * t + 1));
-        a[1] = pack_bf16(ea(g2 + 8, 2 * t), ea(g2 + 8, 2 * t + 1));
-        a[2] = pack_bf16(ea(g2, 2 * t + 8), ea(g2, 2 * t + 9));
-        a[3] = pack_bf16(ea(g2 + 8, 2 * t + 8), ea(g2 + 8, 2 * t + 9));
-        auto eb = [&](int k, int n2) { return k < 8 ? w.w3[k * kH + nt * 8 + n2] : 0.f; };
-        bb[0] = pack_bf16(eb(2 * t, g2), eb(2 * t + 1, g2));
-        bb[1] = pack_bf16(eb(2 * t + 8, g2), eb(2 * t + 9, g2));
-      }
-      mma16816(c, a, bb);
-      store_c(c, b.h2, kH, 0, nt * 8);  // h2 now holds dH2
-    }
-    __syncwarp();
-    // dZ2 = dH2 * (z2 > 0), stored in z2
-    for (int i = lane; i < 16 * kH; i += 32) b.z2[i] = b.z2[i] > 0.f ? b.h2[i] : 0.f;
-    __syncwarp();
-    // dW2 += dZ2^T h1 (64 x 64): A(r, k) = dZ2(k, r), B(k, n) = h1(k, n)
-    for (int mt = 0; mt < kH / 16; ++mt)
-      for (int nt = 0; nt < kH / 8; ++nt) {
-        float c[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t a[4], bb[2];
-        load_a(a, b.z2, 1, kH, mt * 16, 0);
-        load_b(bb, b.h1, kH, 1, 0, nt * 8);
-        mma16816(c, a, bb);
-        const int g2 = lane >> 2, t = lane & 3;
-        atomicAdd(&g[OW2 + (mt * 16 + g2) * kH + nt * 8 + 2 * t], c[0]);
-        atomicAdd(&g[OW2 + (mt * 16 + g2) * kH + nt * 8 + 2 * t + 1], c[1]);
-        atomicAdd(&g[OW2 + (mt * 16 + g2 + 8) * kH + nt * 8 + 2 * t], c[2]);
-        atomicAdd(&g[OW2 + (mt * 16 + g2 + 8) * kH + nt * 8 + 2 * t + 1], c[3]);
-      }
-    for (int c = lane; c < kH; c += 32) {
-      float s = 0.f;
-      for (int r = 0; r < 16; ++r) s += b.z2[r * kH + c];
-      atomicAdd(&g[OB2 + c], s);
-    }
-    // dH1 = dZ2 W2 (16 x 64): A = dZ2 (16 x 64), B(k, n) = w2[k][n]
-    for (int nt = 0; nt < kH / 8; ++nt) {
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
-      for (int kt = 0; kt < kH / 16; ++kt) {
-        uint32_t a[4], bb[2];
-        load_a(a, b.z2, kH, 1, 0, kt * 16);
-        load_b(bb, w.w2, kH, 1, kt * 16, nt * 8);
-        mma16816(c, a, bb);
-      }
-      store_c(c, b.h1, kH, 0, nt * 8);  // h1 now holds dH1
-    }
-    __syncwarp();
-    for (int i = lane; i < 16 * kH; i += 32) b.z1[i] = b.z1[i] > 0.f ? b.h1[i] : 0.f;  // dZ1
-    __syncwarp();
-    // dW1 += dZ1^T x (64 x 16): A(r, k) = dZ1(k, r), B(k, n) = x(k, n)
-    for (int mt = 0; mt < kH / 16; ++mt)
-      for (int nt = 0; nt < 2; ++nt) {
-        float c[4] = {0.f, 0.f, 0.f, 0.f};
-        uint32_t a[4], bb[2];
-        load_a(a, b.z1, 1, kH, mt * 16, 0);
-        load_b(bb, b.x, 16, 1, 0, nt * 8);
-        mma16816(c, a, bb);
-        const int g2 = lane >> 2, t = lane & 3;
-        const int n0 = nt * 8 + 2 * t;
-        if (n0 < kIn) {
-          atomicAdd(&g[OW1 + (mt * 16 + g2) * kIn + n0], c[0]);
-          atomicAdd(&g[OW1 + (mt * 16 + g2 + 8) * kIn + n0], c[2]);
-        }
-        if (n0 + 1 < kIn) {
-          atomicAdd(&g[OW1 + (mt * 16 + g2) * kIn + n0 + 1], c[1]);
-          atomicAdd(&g[OW1 + (mt * 16 + g2 + 8) * kIn + n0 + 1], c[3]);
-        }
-      }
-    for (int c = lane; c < kH; c += 32) {
-      float s = 0.f;
-      for (int r = 0; r < 16; ++r) s += b.z1[r * kH + c];
-      atomicAdd(&g[OB1 + c], s);
-    }
-    __syncwarp();
-  }
-  for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  if (lane == 0) atomicAdd(loss, lsum * inv_n);
-  __syncthreads();
-  for (int i = threadIdx.x; i < kMlpParams; i += blockDim.x) atomicAdd(&grad[i], g[i]);
+// ---- training
+//
+// Shared-memory matrices of the training kernel are BF16, rows padded by 8
+// values: the eight rows of a fragment start in different banks.  ldmatrix
+// reads a fragment, .trans the transposed one, so every matrix is stored once.
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm2(uint32_t (&r)[2], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];"
+               : "=r"(r[0]), "=r"(r[1])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm2t(uint32_t (&r)[2], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
+               : "=r"(r[0]), "=r"(r[1])
+               : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+// Fragments (fragment loaders above define the element places): A (16 x 16 at
+// (r0, k0)) of a matrix stored [r][k], or [k][r] (at); B (16 x 8 at (k0, n0)) of
+// a matrix stored [n][k], or [k][n] (bt).
+__device__ __forceinline__ void frag_a(uint32_t (&a)[4], const __nv_bfloat16* p, int ld, int r0, int k0) {
+  const int lane = threadIdx.x & 31;
+  ldsm4(a, p + (r0 + (lane & 15)) * ld + k0 + (lane >> 4) * 8);
+}
+__device__ __forceinline__ void frag_at(uint32_t (&a)[4], const __nv_bfloat16* p, int ld, int r0, int k0) {
+  const int lane = threadIdx.x & 31;
+  ldsm4t(a, p + (k0 + (lane & 7) + (lane >> 4) * 8) * ld + r0 + ((lane >> 3) & 1) * 8);
+}
+__device__ __forceinline__ void frag_b(uint32_t (&b)[2], const __nv_bfloat16* p, int ld, int k0, int n0) {
+  const int lane = threadIdx.x & 15;
+  ldsm2(b, p + (n0 + (lane & 7)) * ld + k0 + (lane >> 3) * 8);
+}
+__device__ __forceinline__ void frag_bt(uint32_t (&b)[2], const __nv_bfloat16* p, int ld, int k0, int n0) {
+  const int lane = threadIdx.x & 15;
+  ldsm2t(b, p + (k0 + lane) * ld + n0);
+}
+// two values of a C fragment (row, cols n0 + 2t, n0 + 2t + 1)
+__device__ __forceinline__ void put2(__nv_bfloat16* p, int ld, int row, int col, float lo, float hi) {
+  *reinterpret_cast<uint32_t*>(p + row * ld + col) = pack_bf16(lo, hi);
 }
 
-// Adam (Kingma & Ba 2015) on the FP32 master weights.
-__global__ void k_adam(float* __restrict__ prm, const float* __restrict__ grad, float* __restrict__ m1,
-                       float* __restrict__ m2, float lr, float b1, float b2, float eps, float c1, float c2) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= kMlpParams) return;
-  const float g = grad[i];
-  const float a = b1 * m1[i] + (1.f - b1) * g;
-  const float v = b2 * m2[i] + (1.f - b2) * g * g;
-  m1[i] = a;
-  m2[i] = v;
-  prm[i] -= lr * (a / c1) / (sqrtf(v / c2) + eps);
+constexpr int kTrainWarps = 8, kTrainRows = 64;  // warps a CTA, samples of a tile
+constexpr int kLdW = kH + 8, kLdN = 16 + 8;      // row strides of 64- and 16-wide matrices
+static_assert(OW2 % 4 == 0, "16-byte loads of W2");
+static_assert(kH == 8 * kTrainWarps && kIn <= 16 && kOut <= 4, "the tiling of k_mlp_grad");
+struct TrainSmem {
+  __nv_bfloat16 w1[kH * kLdN], w2[kH * kLdW], w3[16 * kLdW];  // [out][in], zero padded
+  __nv_bfloat16 x[kTrainRows * kLdN], dy[kTrainRows * kLdN];  // zero padded
+  __nv_bfloat16 h1[kTrainRows * kLdW], h2[kTrainRows * kLdW], dz1[kTrainRows * kLdW], dz2[kTrainRows * kLdW];
+  float b1[kH], b2[kH], b3[8];
+  int last;
+};
+
+// Adam (Kingma & Ba 2015) on the FP32 master weights, by the last CTA of the
+// gradient kernel; null prm: no update.  done: CTAs that have added their
+// gradient (zero before and after a launch).
+struct AdamStep {
+  float *prm, *m1, *m2;
+  unsigned int* done;
+  float lr, b1, b2, eps, c1, c2;
+};
+
+// Gradient of the mean squared error over the samples idx[0..n) (or 0..n
+// when idx is null), accumulated into grad (kMlpParams) and loss; with an Adam
+// step, the weights' update and grad cleared for the next launch.
+//
+// A mini-batch of thousands of samples is a chain of seven small matrix products,
+// bound by latency.  A CTA takes 64 samples at a time; warp w owns the 8 hidden
+// units [8w, 8w + 8) as columns of every activation and of every weight
+// gradient, so a product is 16 independent mma chains across the CTA, the
+// weight gradients stay in registers over all the tiles of the CTA, and only
+// they meet in atomics, once per CTA.  A batch of 4096 with its Adam step: 18 us;
+// with a tile of 16 samples per warp, every weight gradient of every tile added
+// by shared-memory atomics, and Adam in a launch of its own: 45 + 4 us (ncu).
+__global__ void __launch_bounds__(32 * kTrainWarps)
+    k_mlp_grad(const float* prm, const float* __restrict__ X, const float* __restrict__ T,
+               const int* __restrict__ idx, int n, float* grad, double* loss, AdamStep adam) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  TrainSmem& s = *reinterpret_cast<TrainSmem*>(smem);
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int n0 = 8 * w;
+  const float inv_n = 1.f / (float)n;
+  griddep_launch_dependents();
+  auto sample = [&](int r) -> int64_t { return idx ? idx[r] : r; };
+  auto load_x = [&](int s0) {
+    for (int i = tid; i < kTrainRows * 16; i += blockDim.x) {
+      const int r = i / 16, c = i % 16;
+      s.x[r * kLdN + c] = __float2bfloat16(c < kIn && s0 + r < n ? X[sample(s0 + r) * kIn + c] : 0.f);
+    }
+  };
+  // samples and targets do not come from the launch before this one
+  load_x(blockIdx.x * kTrainRows);
+  for (int i = tid; i < kTrainRows * kLdN; i += blockDim.x) s.dy[i] = __float2bfloat16(0.f);
+  griddep_wait();
+  for (int i = tid; i < kH * 16; i += blockDim.x) {
+    const int r = i / 16, c = i % 16;
+    s.w1[r * kLdN + c] = __float2bfloat16(c < kIn ? __ldcg(prm + OW1 + r * kIn + c) : 0.f);
+  }
+  {
+    float4 v[kH * kH / 4 / (32 * kTrainWarps)];
+#pragma unroll
+    for (int k = 0; k < kH * kH / 4 / (32 * kTrainWarps); ++k)
+      v[k] = __ldcg(reinterpret_cast<const float4*>(prm + OW2) + tid + k * 32 * kTrainWarps);
+#pragma unroll
+    for (int k = 0; k < kH * kH / 4 / (32 * kTrainWarps); ++k) {
+      const int i = 4 * (tid + k * 32 * kTrainWarps);
+      put2(s.w2, kLdW, i / kH, i % kH, v[k].x, v[k].y);
+      put2(s.w2, kLdW, i / kH, i % kH + 2, v[k].z, v[k].w);
+    }
+  }
+  for (int i = tid; i < 16 * kH; i += blockDim.x)
+    s.w3[(i / kH) * kLdW + i % kH] = __float2bfloat16(i < kOut * kH ? __ldcg(prm + OW3 + i) : 0.f);
+  for (int i = tid; i < kH; i += blockDim.x) {
+    s.b1[i] = __ldcg(prm + OB1 + i);
+    s.b2[i] = __ldcg(prm + OB2 + i);
+  }
+  if (tid < 8) s.b3[tid] = tid < kOut ? __ldcg(prm + OB3 + tid) : 0.f;
+  float dw1[4] = {}, dw2[4][4] = {}, dw3[4] = {}, db1[2] = {}, db2[2] = {}, db3[2] = {};
+  double lsum = 0.;
+  for (int s0 = blockIdx.x * kTrainRows; s0 < n; s0 += gridDim.x * kTrainRows) {
+    if (s0 != (int)blockIdx.x * kTrainRows) load_x(s0);
+    __syncthreads();
+    uint32_t a[4], b[2];
+    uint32_t on1 = 0, on2 = 0;  // bit 4 mt + c: the unit of C element c is active
+    // h1 = relu(x w1^T + b1)
+    frag_b(b, s.w1, kLdN, 0, n0);
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt) {
+      float c[4] = {0.f, 0.f, 0.f, 0.f};
+      frag_a(a, s.x, kLdN, 16 * mt, 0);
+      mma16816(c, a, b);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        c[k] += s.b1[n0 + 2 * t + (k & 1)];
+        on1 |= (c[k] > 0.f ? 1u : 0u) << (4 * mt + k);
+        c[k] = fmaxf(c[k], 0.f);
+      }
+      put2(s.h1, kLdW, 16 * mt + g, n0 + 2 * t, c[0], c[1]);
+      put2(s.h1, kLdW, 16 * mt + g + 8, n0 + 2 * t, c[2], c[3]);
+    }
+    __syncthreads();
+    // h2 = relu(h1 w2^T + b2)
+    {
+      float c[4][4] = {};
+#pragma unroll
+      for (int kt = 0; kt < 4; ++kt) {
+        frag_b(b, s.w2, kLdW, 16 * kt, n0);
+#pragma unroll
+        for (int mt = 0; mt < 4; ++mt) {
+          frag_a(a, s.h1, kLdW, 16 * mt, 16 * kt);
+          mma16816(c[mt], a, b);
+        }
+      }
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          c[mt][k] += s.b2[n0 + 2 * t + (k & 1)];
+          on2 |= (c[mt][k] > 0.f ? 1u : 0u) << (4 * mt + k);
+          c[mt][k] = fmaxf(c[mt][k], 0.f);
+        }
+        put2(s.h2, kLdW, 16 * mt + g, n0 + 2 * t, c[mt][0], c[mt][1]);
+        put2(s.h2, kLdW, 16 * mt + g + 8, n0 + 2 * t, c[mt][2], c[mt][3]);
+      }
+    }
+    __syncthreads();
+    // y = h2 w3^T + b3 and dL/dy = 2 (y - t) / n: one row tile each of warps 0 - 3
+    if (w < 4) {
+      float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int kt = 0; kt < 4; ++kt) {
+        frag_a(a, s.h2, kLdW, 16 * w, 16 * kt);
+        frag_b(b, s.w3, kLdW, 16 * kt, 0);
+        mma16816(c, a, b);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int col = 2 * t + (k & 1), row = 16 * w + g + 8 * (k >> 1);
+        float d = 0.f;
+        if (col < kOut && s0 + row < n) {
+          const float e = c[k] + s.b3[col] - T[sample(s0 + row) * kOut + col];
+          lsum += (double)e * e;
+          d = 2.f * e * inv_n;
+        }
+        db3[k & 1] += d;
+        c[k] = d;
+      }
+      put2(s.dy, kLdN, 16 * w + g, 2 * t, c[0], c[1]);
+      put2(s.dy, kLdN, 16 * w + g + 8, 2 * t, c[2], c[3]);
+    }
+    __syncthreads();
+    // dz2 = (dy w3) where z2 > 0; dw3 += dy^T h2
+    frag_bt(b, s.w3, kLdW, 0, n0);
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt) {
+      float c[4] = {0.f, 0.f, 0.f, 0.f};
+      frag_a(a, s.dy, kLdN, 16 * mt, 0);
+      mma16816(c, a, b);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (!(on2 >> (4 * mt + k) & 1)) c[k] = 0.f;
+        db2[k & 1] += c[k];
+      }
+      put2(s.dz2, kLdW, 16 * mt + g, n0 + 2 * t, c[0], c[1]);
+      put2(s.dz2, kLdW, 16 * mt + g + 8, n0 + 2 * t, c[2], c[3]);
+    }
+#pragma unroll
+    for (int kt = 0; kt < 4; ++kt) {
+      frag_at(a, s.dy, kLdN, 0, 16 * kt);
+      frag_bt(b, s.h2, kLdW, 16 * kt, n0);
+      mma16816(dw3, a, b);
+    }
+    __syncthreads();
+    // dz1 = (dz2 w2) where z1 > 0; dw2 += dz2^T h1
+    {
+      float c[4][4] = {};
+#pragma unroll
+      for (int kt = 0; kt < 4; ++kt) {
+        frag_bt(b, s.w2, kLdW, 16 * kt, n0);
+#pragma unroll
+        for (int mt = 0; mt < 4; ++mt) {
+          frag_a(a, s.dz2, kLdW, 16 * mt, 16 * kt);
+          mma16816(c[mt], a, b);
+        }
+      }
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (!(on1 >> (4 * mt + k) & 1)) c[mt][k] = 0.f;
+          db1[k & 1] += c[mt][k];
+        }
+        put2(s.dz1, kLdW, 16 * mt + g, n0 + 2 * t, c[mt][0], c[mt][1]);
+        put2(s.dz1, kLdW, 16 * mt + g + 8, n0 + 2 * t, c[mt][2], c[mt][3]);
+      }
+#pragma unroll
+      for (int kt = 0; kt < 4; ++kt) {
+        frag_bt(b, s.h1, kLdW, 16 * kt, n0);
+#pragma unroll
+        for (int mt = 0; mt < 4; ++mt) {
+          frag_at(a, s.dz2, kLdW, 16 * mt, 16 * kt);
+          mma16816(dw2[mt], a, b);
+        }
+      }
+    }
+    __syncthreads();
+    // dw1 += dz1^T x: one 16 x 8 tile of it a warp
+#pragma unroll
+    for (int kt = 0; kt < 4; ++kt) {
+      frag_at(a, s.dz1, kLdW, 16 * (w & 3), 16 * kt);
+      frag_bt(b, s.x, kLdN, 16 * kt, 8 * (w >> 2));
+      mma16816(dw1, a, b);
+    }
+    __syncthreads();  // the next tile overwrites x
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int row = g + 8 * (k >> 1), col = 2 * t + (k & 1);
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt) atomicAdd(grad + OW2 + (16 * mt + row) * kH + n0 + col, dw2[mt][k]);
+    if (8 * (w >> 2) + col < kIn)
+      atomicAdd(grad + OW1 + (16 * (w & 3) + row) * kIn + 8 * (w >> 2) + col, dw1[k]);
+    if (row < kOut) atomicAdd(grad + OW3 + row * kH + n0 + col, dw3[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) {
+      db1[k] += __shfl_xor_sync(0xffffffffu, db1[k], o);
+      db2[k] += __shfl_xor_sync(0xffffffffu, db2[k], o);
+      db3[k] += __shfl_xor_sync(0xffffffffu, db3[k], o);
+    }
+    if (g == 0) {
+      atomicAdd(grad + OB1 + n0 + 2 * t + k, db1[k]);
+      atomicAdd(grad + OB2 + n0 + 2 * t + k, db2[k]);
+      if (w < 4 && 2 * t + k < kOut) atomicAdd(grad + OB3 + 2 * t + k, db3[k]);
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+  if (lane == 0 && w < 4) atomicAdd(loss, lsum * inv_n);
+  if (!adam.prm) return;
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s.last = atomicAdd(adam.done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s.last) return;
+  __threadfence();
+  auto update = [&](float d, float& m1, float& m2, float& p) {
+    const float m = adam.b1 * m1 + (1.f - adam.b1) * d;
+    const float v = adam.b2 * m2 + (1.f - adam.b2) * d * d;
+    m1 = m;
+    m2 = v;
+    p -= adam.lr * (m / adam.c1) / (sqrtf(v / adam.c2) + adam.eps);
+  };
+  // four parameters a load, every load of the thread in flight
+  constexpr int kQuads = kMlpParams / 4, kRounds = (kQuads + 32 * kTrainWarps - 1) / (32 * kTrainWarps);
+  float4 d4[kRounds], m4[kRounds], v4[kRounds], p4[kRounds];
+#pragma unroll
+  for (int k = 0; k < kRounds; ++k) {
+    const int i = tid + k * 32 * kTrainWarps;
+    if (i < kQuads) {
+      d4[k] = __ldcg(reinterpret_cast<const float4*>(grad) + i);
+      m4[k] = __ldcg(reinterpret_cast<const float4*>(adam.m1) + i);
+      v4[k] = __ldcg(reinterpret_cast<const float4*>(adam.m2) + i);
+      p4[k] = __ldcg(reinterpret_cast<const float4*>(adam.prm) + i);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < kRounds; ++k) {
+    const int i = tid + k * 32 * kTrainWarps;
+    if (i < kQuads) {
+      update(d4[k].x, m4[k].x, v4[k].x, p4[k].x);
+      update(d4[k].y, m4[k].y, v4[k].y, p4[k].y);
+      update(d4[k].z, m4[k].z, v4[k].z, p4[k].z);
+      update(d4[k].w, m4[k].w, v4[k].w, p4[k].w);
+      reinterpret_cast<float4*>(adam.m1)[i] = m4[k];
+      reinterpret_cast<float4*>(adam.m2)[i] = v4[k];
+      reinterpret_cast<float4*>(adam.prm)[i] = p4[k];
+      reinterpret_cast<float4*>(grad)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  if (4 * kQuads + tid < kMlpParams) {
+    const int i = 4 * kQuads + tid;
+    update(__ldcg(grad + i), adam.m1[i], adam.m2[i], adam.prm[i]);
+    grad[i] = 0.f;
+  }
+  if (tid == 0) *adam.done = 0u;
 }
 
 #define CKM(x)                                                                                      \
@@ -377,9 +547,7 @@ __global__ void k_adam(float* __restrict__ prm, const float* __restrict__ grad, 
 
 constexpr int kMlpThreads = 128;  // 4 warps
 size_t fwd_smem() { return sizeof(SmemWeights) + 4 * sizeof(WarpBuf); }
-size_t grad_smem() {
-  return sizeof(SmemWeights) + sizeof(float) * ((kMlpParams + 63) / 64 * 64) + 4 * sizeof(WarpBuf);
-}
+size_t grad_smem() { return sizeof(TrainSmem); }
 
 template <typename T>
 struct DBuf {
@@ -417,19 +585,17 @@ void mlp_forward_counted(const float* prm, const float* X, const int* n_dev, int
   k_mlp_forward<<<grid, kMlpThreads, fwd_smem(), st>>>(prm, X, cap, n_dev, Y);
 }
 
+static void launch_grad(const float* prm, const float* X, const float* T, const int* idx, int n, float* grad,
+                        double* loss, const AdamStep& adam, cudaStream_t st) {
+  ensure_smem_attrs();
+  const int grid = std::min(148 * 2, (n + kTrainRows - 1) / kTrainRows);
+  launch_dependent(k_mlp_grad, grid, 32 * kTrainWarps, grad_smem(), st, prm, X, T, idx, n, grad, loss, adam);
+}
+
 void mlp_grad_device(const float* prm, const float* X, const float* T, const int* idx, int n, float* grad,
                      double* loss, cudaStream_t st) {
   if (n <= 0) return;
-  ensure_smem_attrs();
-  const int grid = std::min(148 * 2, (n + 63) / 64);
-  k_mlp_grad<<<grid, kMlpThreads, grad_smem(), st>>>(prm, X, T, idx, n, grad, loss);
-}
-
-
-void mlp_adam_device(float* prm, const float* grad, float* m1, float* m2, double lr, int64_t step, cudaStream_t st) {
-  const double b1 = 0.9, b2 = 0.999;
-  const float c1 = (float)(1. - std::pow(b1, (double)step)), c2 = (float)(1. - std::pow(b2, (double)step));
-  k_adam<<<(kMlpParams + 255) / 256, 256, 0, st>>>(prm, grad, m1, m2, (float)lr, (float)b1, (float)b2, 1e-8f, c1, c2);
+  launch_grad(prm, X, T, idx, n, grad, loss, AdamStep{}, st);
 }
 
 double mlp_train_device(float* prm, const float* X, const float* T, int n, int epochs, int batch, double lr,
@@ -444,6 +610,9 @@ double mlp_train_device(float* prm, const float* X, const float* T, int n, int e
   DBuf<float> dg(kMlpParams), m1(kMlpParams), m2(kMlpParams);
   DBuf<double> dl(1);
   DBuf<int> didx(n);
+  DBuf<unsigned int> done(1);
+  CKM(cudaMemsetAsync(dg.p, 0, kMlpParams * sizeof(float), st));
+  CKM(cudaMemsetAsync(done.p, 0, sizeof(unsigned int), st));
   CKM(cudaMemsetAsync(m1.p, 0, kMlpParams * sizeof(float), st));
   CKM(cudaMemsetAsync(m2.p, 0, kMlpParams * sizeof(float), st));
   int64_t step = 0;
@@ -456,9 +625,11 @@ double mlp_train_device(float* prm, const float* X, const float* T, int n, int e
     int nbatches = 0;
     for (int s0 = 0; s0 < ntr; s0 += batch) {
       const int nb = std::min(batch, ntr - s0);
-      CKM(cudaMemsetAsync(dg.p, 0, kMlpParams * sizeof(float), st));
-      mlp_grad_device(prm, X, T, didx.p + s0, nb, dg.p, dl.p, st);
-      mlp_adam_device(prm, dg.p, m1.p, m2.p, lr, ++step, st);
+      const double b1 = 0.9, b2 = 0.999;
+      ++step;
+      const AdamStep adam{prm,       m1.p,      m2.p, done.p, (float)lr, (float)b1, (float)b2, 1e-8f,
+                          (float)(1. - std::pow(b1, (double)step)), (float)(1. - std::pow(b2, (double)step))};
+      launch_grad(prm, X, T, didx.p + s0, nb, dg.p, dl.p, adam, st);
       ++nbatches;
     }
     double sum = 0.;

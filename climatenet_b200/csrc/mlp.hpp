@@ -20,9 +20,6 @@ void mlp_forward_counted(const float* prm, const float* X, const int* n_dev, int
 // idx is null) into grad and the loss into *loss (both must be zeroed first).
 void mlp_grad_device(const float* prm, const float* X, const float* T, const int* idx, int n, float* grad,
                      double* loss, cudaStream_t st);
-// Adam on device: step is the 1-based update count.
-void mlp_adam_device(float* prm, const float* grad, float* m1, float* m2, double lr, int64_t step, cudaStream_t st);
-
 // Trains prm (device, in place) on the n samples X (n x 10), T (n x 3), both
 // device-resident: seeded shuffle, 90/10 split, `epochs` passes of Adam over
 // the training part in mini-batches.  Returns the mean training loss of the

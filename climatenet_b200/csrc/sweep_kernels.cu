@@ -107,16 +107,6 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }
 __device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-// Programmatic dependent launch: a kernel launched with the programmatic
-// stream serialization attribute may start while the kernel before it in the
-// stream still runs; griddep_wait() returns once that kernel has completed
-// and its memory operations are visible.  Before it, such a kernel reads
-// only data no kernel of the solve writes (the factor, the plan).
-// griddep_launch_dependents() lets the next such kernel start launching.
-__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void griddep_launch_dependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 // orders generic-proxy accesses of shared memory before the bulk copies that
 // follow (a slot's earlier reads before the copy that overwrites it)
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -1147,24 +1137,6 @@ bool configure_solve(DPlan& P, int shape) {
   P.grid_lf = resident_ctas(level_kernel<T, true>(P.chunk), level, 32 * kLevelWarps);
   P.grid_lb = resident_ctas(level_kernel<T, false>(P.chunk), level, 32 * kLevelWarps);
   return rf > 0 && rb > 0 && P.grid_lf > 0 && P.grid_lb > 0;
-}
-
-// Launch as a programmatic dependent of the previous kernel in the stream
-// (the kernel calls griddep_wait() before it reads what that kernel writes).
-template <typename... Params, typename... Args>
-void launch_dependent(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t st,
-                      Args&&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
 template <typename T>

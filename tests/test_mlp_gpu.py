@@ -231,3 +231,25 @@ def test_handle_trains_on_its_own_log():
     Y = native.mlp_forward(w, X)
     r2 = 1.0 - ((Y - T) ** 2).sum() / ((T - T.mean(0)) ** 2).sum()
     assert r2 > 0.4
+
+
+@pytest.mark.parametrize("n", [1, 15, 64, 65, 130, 1000, 2 * 148 * 64 + 65])
+def test_gradient_is_the_mean_over_any_split(n):
+    """The training kernel's tiles hold 64 samples and its grid 2 x 148 of them:
+    the gradient of n samples is the weighted mean of the gradients of its parts.
+    Each sample's output gradient is rounded to BF16 (2^-9 relative) after its
+    scaling by 2 / n, so the two sides agree to 2^-8 of the norm."""
+    rng = np.random.default_rng(n)
+    X = rng.standard_normal((n, abi.MLP_IN)).astype(np.float32)
+    T = rng.standard_normal((n, abi.MLP_OUT)).astype(np.float32)
+    w = native.mlp_init(2)
+    w[-abi.MLP_OUT * (abi.MLP_HIDDEN + 1):] *= 10
+    loss, g = native.mlp_gradient(w, X, T)
+    cuts = sorted({0, n, n // 3, min(n, 37), max(0, n - 9)})
+    ml, mg = 0.0, np.zeros_like(g, dtype=np.float64)
+    for a, b in zip(cuts[:-1], cuts[1:]):
+        pl, pg = native.mlp_gradient(w, X[a:b], T[a:b])
+        ml += pl * (b - a) / n
+        mg += pg.astype(np.float64) * (b - a) / n
+    assert abs(loss - ml) <= 1e-5 * ml
+    assert np.linalg.norm(g - mg) <= 2.0 ** -8 * np.linalg.norm(mg)
