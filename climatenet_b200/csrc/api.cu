@@ -59,7 +59,7 @@ constexpr int kStrideBlocks = 592;  // 4 x 148 SMs for grid-stride kernels
 // Work items of the upper supernodes are at most 32 x chunk elements and the
 // subtree blocks reach up to the cut level; both are chosen per scene by the
 // autotuner in create_impl among these.
-constexpr int kChunk = 64;
+constexpr int kChunk = 32;  // first stage of the autotuner: the best width nearly everywhere
 constexpr int kCutLevel = 4;  // host emulation check (pdf_factor_check)
 constexpr int kRecords = 64;  // step records in flight before the oldest is harvested
 constexpr int kChunkCandidates[3] = {32, 64, 128};

@@ -107,10 +107,8 @@ constexpr int kMaxBlockLevels = 16;
 constexpr int kMaxBlockCols = 1536;
 constexpr int kMaxBlockExt = 1024;
 constexpr int kMaxBlockItems = 768;  // work items per block and sweep (staged in shared memory)
-// columns (forward) / rows (backward) per bulk copy: 16 in FP64, 32 in FP32
-// (4 KB either way); item starts and the backward index lists are aligned to
-// the larger
-constexpr int kSlab = 16;
+// columns (forward) / rows (backward) per bulk copy; item starts and the
+// backward index lists are aligned to it
 constexpr int kSlabMax = 32;
 // A tile longer than its sweep's span (forward columns, backward rows) is
 // split into items of that span whose partial sums meet in atomics, so that

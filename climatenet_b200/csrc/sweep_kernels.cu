@@ -59,16 +59,13 @@ constexpr int kSweepThreads = 256;
 constexpr int kBlockMaxThreads = 576;
 
 // A slab (one bulk copy) is 32 rows x kCols columns (forward) or kCols rows
-// x 32 columns (backward): 4 KB, except FP32 backward slabs of 16 rows (2 KB,
-// measured faster there: the per-row index staging is half as long).  A
-// block kernel's CTA has a ring of R slots (DPlan::ring_f / ring_b): the
-// largest in [kMinSlots, kMaxSlots] with which the launch shape's CTAs fit an
-// SM.
-template <typename T, bool kFwd>
-struct Stages {
-  static constexpr int kCols = (sizeof(T) == 4 && kFwd) ? kSlabMax : kSlab;
-  static constexpr int kElems = kTile * kCols;
-};
+// x 32 columns (backward): 8 KB in FP64, 4 KB in FP32.  (With 16 the wait for a
+// slab and the staging of its vector entries weigh twice: 500 x 500 cloth, FP64
+// forward 55 us instead of 48, FP32 backward 68 instead of 53.)  A block kernel's
+// CTA has a ring of R slots (DPlan::ring_f / ring_b): the largest in [kMinSlots,
+// kMaxSlots] with which the launch shape's CTAs fit an SM.
+constexpr int kCols = kSlabMax;
+constexpr int kSlabElems = kTile * kCols;
 constexpr int kMinSlots = 4, kMaxSlots = 64;
 
 __device__ __forceinline__ unsigned long long ld_volatile_u64(const unsigned long long* p) {
@@ -197,7 +194,7 @@ __device__ __forceinline__ void stage_items(BlockItem* dst, const BlockItem* src
 // the ring's parts in shared memory
 template <typename T>
 struct BlockSmem {
-  T* ring;          // R slots of Stages::kElems
+  T* ring;          // R slots of kSlabElems
   int* iring;       // backward: R slots of kCols row indices
   uint64_t* full;   // R
   uint64_t* empty;  // R
@@ -212,7 +209,7 @@ struct BlockSmem {
 template <typename T, bool kFwd>
 __device__ __forceinline__ BlockSmem<T> block_smem(unsigned char* base, int ncw, int warp, int max_ld, int max_cols,
                                                    int max_items, int R) {
-  constexpr int KE = Stages<T, kFwd>::kElems, kCols = Stages<T, kFwd>::kCols;
+  constexpr int KE = kSlabElems;
   BlockSmem<T> s;
   size_t off = 0;
   s.ring = reinterpret_cast<T*>(base);
@@ -239,7 +236,7 @@ __device__ __forceinline__ BlockSmem<T> block_smem(unsigned char* base, int ncw,
 
 template <typename T, bool kFwd>
 size_t block_smem_bytes(int ncw, int max_ld, int max_cols, int max_items, int R) {
-  constexpr int KE = Stages<T, kFwd>::kElems, kCols = Stages<T, kFwd>::kCols;
+  constexpr int KE = kSlabElems;
   size_t b = (size_t)R * KE * sizeof(T) + 3 * (size_t)R * sizeof(uint64_t) + 3 * (size_t)max_ld * sizeof(T);
   if (!kFwd) b += (size_t)R * kCols * sizeof(int) + 3 * (size_t)max_cols * sizeof(T) + (size_t)ncw * 3 * kCols * sizeof(T);
   return ((b + 15) & ~size_t(15)) + (size_t)max_items * (sizeof(BlockItem) + sizeof(int));
@@ -272,7 +269,6 @@ __device__ __forceinline__ void consumers_sync(int nthreads) {
 
 // Warp 0: slab0[k] = the number of slabs of items [0, k) (kCols columns /
 // rows each, from a0); returns the total (every lane).
-template <int kCols>
 __device__ __forceinline__ int scan_slabs(const BlockItem* items, int nitems, int* slab0, int lane) {
   int total = 0;
   for (int k0 = 0; k0 < nitems; k0 += 32) {
@@ -296,7 +292,7 @@ __device__ __forceinline__ int scan_slabs(const BlockItem* items, int nitems, in
 template <typename T, bool kFwd>
 __device__ __forceinline__ int produce_block(const BlockSmem<T>& sm, const BlockItem* items, int nitems, int q_base,
                                              int R, const T* W, const int* bidx, int max_spins, bool& ok) {
-  constexpr int KE = Stages<T, kFwd>::kElems, kCols = Stages<T, kFwd>::kCols;
+  constexpr int KE = kSlabElems;
   int q = q_base;
   for (int it = 0; it < nitems; ++it) {
     const BlockItem I = items[it];
@@ -334,7 +330,7 @@ __global__ void __launch_bounds__(kBlockMaxThreads, 1) k_block_forward(DPlan P, 
                                                                     int n, SweepSync sy) {
   trace_stamp(sy.trace, DTrace::kSolve);
   griddep_launch_dependents();  // the first upper level may start on SMs this sweep leaves
-  constexpr int KE = Stages<T, true>::kElems, kCols = Stages<T, true>::kCols;
+  constexpr int KE = kSlabElems;
   const int R = P.ring_f;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int s_ticket, s_nslab, s_failed;
@@ -382,7 +378,7 @@ __global__ void __launch_bounds__(kBlockMaxThreads, 1) k_block_forward(DPlan P, 
     cp_async_wait_all();
     __syncthreads();
     if (warp == 0) {
-      const int t = scan_slabs<kCols>(sm.items, nitems, sm.slab0, lane);
+      const int t = scan_slabs(sm.items, nitems, sm.slab0, lane);
       if (lane == 0) s_nslab = t;
     }
     __syncthreads();
@@ -527,7 +523,7 @@ __global__ void __launch_bounds__(kBlockMaxThreads, 1) k_block_backward(DPlan P,
                                                                      const T* __restrict__ y, const T* x, int n,
                                                                      SweepSync sy, WriteBack wb) {
   griddep_launch_dependents();
-  constexpr int KE = Stages<T, false>::kElems, kCols = Stages<T, false>::kCols;
+  constexpr int KE = kSlabElems;
   const int R = P.ring_b;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ int s_ticket, s_nslab, s_failed;
@@ -596,7 +592,7 @@ __global__ void __launch_bounds__(kBlockMaxThreads, 1) k_block_backward(DPlan P,
     cp_async_wait_all();
     __syncthreads();
     if (warp == 0) {
-      const int t = scan_slabs<kCols>(sm.items, nitems, sm.slab0, lane);
+      const int t = scan_slabs(sm.items, nitems, sm.slab0, lane);
       if (lane == 0) s_nslab = t;
     }
     __syncthreads();
