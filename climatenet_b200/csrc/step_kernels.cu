@@ -269,7 +269,7 @@ template void launch_friction_obstacle<float>(dim3, dim3, cudaStream_t, DModel, 
 // SMs take part.  A cluster gives 16 of them with a hardware barrier between
 // the phases; a whole-device barrier would cost more than the passes it saves
 // below some 16k contacts a level.  One iteration of 7.3k contacts in 3 levels:
-// 32 us, against 146 us on one CTA of 1024 threads; of 11.5k contacts: 33 us
+// 27 us, against 146 us on one CTA of 1024 threads; of 11.5k contacts: 28 us
 // against 185 us; without contacts 4 us either way (ncu).
 // The forces sf change between phases on other SMs: they are read past L1.
 constexpr int kSelfCtas = 16, kSelfThreads = 512;
@@ -281,6 +281,58 @@ __device__ __forceinline__ double3 ld3cg(const double* p, int64_t i) {
   return make_double3(__ldcg(p + 3 * i), __ldcg(p + 3 * i + 1), __ldcg(p + 3 * i + 2));
 }
 
+// What a self contact's estimate reads that no phase changes.
+struct SelfRec {
+  int sc, sa, sb;          // contact, slots of its vertices
+  double B[9], mA, mB, mu;
+  double3 fa, fb, rem;     // f + contact force at the slots, the contact's force of the last iteration
+};
+__device__ __forceinline__ void self_fetch(SelfRec& r, const DModel& m, const DContacts& c, int nxt, int i) {
+  r.sc = c.level_order[i];
+  r.sa = c.s_slota[r.sc];
+  r.sb = c.s_slotb[r.sc];
+  r.mA = m.mass[c.s_vertex[r.sc]];
+  r.mB = m.mass[c.s_partner[r.sc]];
+  r.mu = c.s_mu[r.sc];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) r.B[k] = c.s_basis[9 * (int64_t)r.sc + k];
+  r.rem = ld3(c.s_remember, r.sc);
+  r.fa = ld3(c.f, r.sa) + ld3(c.cf[nxt], r.sa);
+  r.fb = ld3(c.f, r.sb) + ld3(c.cf[nxt], r.sb);
+}
+__device__ __forceinline__ double3 self_estimate(const SelfRec& r, const DContacts& c, int cur, int nxt) {
+  const double3 fA = r.fa + ld3cg(c.sf[cur], r.sa) + ld3cg(c.sf[nxt], r.sa) - r.rem;
+  const double3 fB = r.fb + ld3cg(c.sf[cur], r.sb) + ld3cg(c.sf[nxt], r.sb) + r.rem;
+  const double ia = 1. / r.mA, ib = 1. / r.mB;
+  const double3 fl =
+      basis_t(r.B, make_double3(ia * fA.x - ib * fB.x, ia * fA.y - ib * fB.y, ia * fA.z - ib * fB.z));
+  if (fl.x > 0.) return make_double3(0., 0., 0.);
+  double3 f = cone_project(fl, r.mu);
+  const double sc2 = (r.mA * r.mB) / (r.mA + r.mB);
+  f = make_double3(sc2 * f.x, sc2 * f.y, sc2 * f.z);
+  st3(c.s_force, r.sc, f);
+  return basis_v(r.B, f);
+}
+__device__ __forceinline__ void self_update(const DContacts& c, int cur, int nxt, int sc, int sa, int sb, double3 prev,
+                                            double3 g) {
+  atomicAdd(c.sf[cur] + 3 * sa, -prev.x);
+  atomicAdd(c.sf[cur] + 3 * sa + 1, -prev.y);
+  atomicAdd(c.sf[cur] + 3 * sa + 2, -prev.z);
+  atomicAdd(c.sf[cur] + 3 * sb, prev.x);
+  atomicAdd(c.sf[cur] + 3 * sb + 1, prev.y);
+  atomicAdd(c.sf[cur] + 3 * sb + 2, prev.z);
+  atomicAdd(c.sf[nxt] + 3 * sa, g.x);
+  atomicAdd(c.sf[nxt] + 3 * sa + 1, g.y);
+  atomicAdd(c.sf[nxt] + 3 * sa + 2, g.z);
+  atomicAdd(c.sf[nxt] + 3 * sb, -g.x);
+  atomicAdd(c.sf[nxt] + 3 * sb + 1, -g.y);
+  atomicAdd(c.sf[nxt] + 3 * sb + 2, -g.z);
+  st3(c.s_remember, sc, g);
+}
+
+// A thread's first contact of a level stays in registers from its estimate to
+// its update, and the next level's is fetched before the barrier that opens it,
+// so that a phase begins with the loads of sf alone.
 template <typename T>
 __global__ void __launch_bounds__(kSelfThreads)
     k_friction_self(DModel m, DContacts c, T* __restrict__ b, double* __restrict__ newf, const int* __restrict__ iter) {
@@ -292,50 +344,38 @@ __global__ void __launch_bounds__(kSelfThreads)
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
   if (S > 0) {
     const int nl = *c.n_levels;
-    for (int l = 0; l < nl; ++l) {
-      const int l0 = c.level_ptr[l], l1 = c.level_ptr[l + 1];
-      if (l0 == l1) continue;
-      for (int i = l0 + t0; i < l1; i += step) {
-        const int sc = c.level_order[i];
-        const int sa = c.s_slota[sc], sb = c.s_slotb[sc];
-        const int va = c.s_vertex[sc], vb = c.s_partner[sc];
-        const double* Bm = c.s_basis + 9 * (int64_t)sc;
-        const double mA = m.mass[va], mB = m.mass[vb];
-        const double3 rem = ld3(c.s_remember, sc);
-        const double3 fA = ld3(c.f, sa) + ld3(c.cf[nxt], sa) + ld3cg(c.sf[cur], sa) + ld3cg(c.sf[nxt], sa) - rem;
-        const double3 fB = ld3(c.f, sb) + ld3(c.cf[nxt], sb) + ld3cg(c.sf[cur], sb) + ld3cg(c.sf[nxt], sb) + rem;
-        const double ia = 1. / mA, ib = 1. / mB;
-        const double3 fl = basis_t(Bm, make_double3(ia * fA.x - ib * fB.x, ia * fA.y - ib * fB.y, ia * fA.z - ib * fB.z));
-        double3 g = make_double3(0., 0., 0.);
-        if (!(fl.x > 0.)) {
-          double3 r = cone_project(fl, c.s_mu[sc]);
-          const double sc2 = (mA * mB) / (mA + mB);
-          r = make_double3(sc2 * r.x, sc2 * r.y, sc2 * r.z);
-          st3(c.s_force, sc, r);
-          g = basis_v(Bm, r);
-        }
-        st3(newf, sc, g);
+    int l = 0, l0 = 0, l1 = 0;
+    bool has = false;
+    SelfRec r;
+    // the next level with contacts, this thread's first one fetched; false after the last
+    auto open = [&]() {
+      for (; l < nl; ++l) {
+        l0 = c.level_ptr[l];
+        l1 = c.level_ptr[l + 1];
+        if (l0 == l1) continue;
+        has = l0 + t0 < l1;
+        if (has) self_fetch(r, m, c, nxt, l0 + t0);
+        ++l;
+        return true;
+      }
+      return false;
+    };
+    bool more = open();
+    while (more) {
+      double3 g = make_double3(0., 0., 0.);
+      if (has) g = self_estimate(r, c, cur, nxt);
+      for (int i = l0 + t0 + step; i < l1; i += step) {
+        SelfRec q;
+        self_fetch(q, m, c, nxt, i);
+        st3(newf, q.sc, self_estimate(q, c, cur, nxt));
       }
       cluster_sync();
-      for (int i = l0 + t0; i < l1; i += step) {
+      if (has) self_update(c, cur, nxt, r.sc, r.sa, r.sb, r.rem, g);
+      for (int i = l0 + t0 + step; i < l1; i += step) {
         const int sc = c.level_order[i];
-        const int sa = c.s_slota[sc], sb = c.s_slotb[sc];
-        const double3 prev = ld3(c.s_remember, sc);
-        const double3 g = ld3(newf, sc);
-        atomicAdd(c.sf[cur] + 3 * sa, -prev.x);
-        atomicAdd(c.sf[cur] + 3 * sa + 1, -prev.y);
-        atomicAdd(c.sf[cur] + 3 * sa + 2, -prev.z);
-        atomicAdd(c.sf[cur] + 3 * sb, prev.x);
-        atomicAdd(c.sf[cur] + 3 * sb + 1, prev.y);
-        atomicAdd(c.sf[cur] + 3 * sb + 2, prev.z);
-        atomicAdd(c.sf[nxt] + 3 * sa, g.x);
-        atomicAdd(c.sf[nxt] + 3 * sa + 1, g.y);
-        atomicAdd(c.sf[nxt] + 3 * sa + 2, g.z);
-        atomicAdd(c.sf[nxt] + 3 * sb, -g.x);
-        atomicAdd(c.sf[nxt] + 3 * sb + 1, -g.y);
-        atomicAdd(c.sf[nxt] + 3 * sb + 2, -g.z);
-        st3(c.s_remember, sc, g);
+        self_update(c, cur, nxt, sc, c.s_slota[sc], c.s_slotb[sc], ld3(c.s_remember, sc), ld3(newf, sc));
       }
+      more = open();
       cluster_sync();
     }
   }
