@@ -811,10 +811,10 @@ void launch_iteration(pdf_handle* h, T* b, T* y, T* x, const T* Wf, const T* Wb,
 }
 
 // Kernels of this library launched by one PD iteration (CUB's not counted):
-// [bending], vertex rhs, friction, [self friction], forward, backward, post (small
+// [bending], vertex rhs, friction, [self friction], forward, backward (small
 // scenes: one product), AC.
 int64_t launches_per_iteration(const pdf_handle* h) {
-  return (h->d.dense ? 4 : 6) + (h->dm.B > 0 ? 1 : 0) + (h->prm.self_collision ? 1 : 0);
+  return (h->d.dense ? 4 : 5) + (h->dm.B > 0 ? 1 : 0) + (h->prm.self_collision ? 1 : 0);
 }
 
 // Per step outside the iterations: predictor, obstacle flags + clamp + materialise,

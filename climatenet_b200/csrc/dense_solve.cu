@@ -34,7 +34,7 @@ __device__ __forceinline__ void dot16(double2 w, const double* b, double& s0, do
   s1 += w.y * v.y;
 }
 
-// x = inv(A) b, with the write-back of v and q^k (as k_solve_post).  One warp a
+// x = inv(A) b, with the write-back of v and q^k (as the sweeps').  One warp a
 // row, 16 bytes a lane and load, b of the whole scene in shared memory (each
 // component from a 16-byte boundary, zero between them, as the rows' padding is).
 // Bound by the launch and a few memory latencies for cloths of some hundred

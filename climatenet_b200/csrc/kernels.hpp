@@ -184,9 +184,9 @@ void launch_friction_self(cudaStream_t st, DModel m, DContacts c, T* b, double* 
 cudaError_t configure_friction_self();  // before its first launch on a device
 // Solve vectors b, y, x are three planes of n values (x, y, z components) in
 // pivot order.  y and x of the upper supernodes must be zero before a solve
-// (the previous solve's write-back, or launch_solve_prep).  One solve is the
-// forward sweep, the backward sweep (with the blocks' write-back) and the
-// write-back of the upper columns.
+// (the previous solve's backward and this one's forward block kernel see to
+// that, or launch_solve_prep).  One solve is the forward and the backward sweep,
+// the last kernel of which writes v and q^k back.
 template <typename T>
 bool configure_solve(DPlan& P, int shape);  // shared memory and grids; false if the shape does not fit
 template <typename T>

@@ -35,7 +35,7 @@
 //     of their ext rows are loaded into shared memory, the factor and, per
 //     slab, the row-index list of the tile stream in as in launch 1, and x of
 //     the block's columns is written back into v and q^k directly.
-//  5. k_solve_post — the write-back of the upper supernodes' columns.
+//     The CTAs that run out of blocks write back the upper supernodes' columns.
 // The launches after the first are programmatic dependents of the one before
 // them (griddepcontrol).  Completion counters are cumulative over solves:
 // supernode s has finished solve number e when its counter reaches e * (its
@@ -325,9 +325,60 @@ __device__ __forceinline__ void drain_ring(uint64_t* full, int q_end, int R, int
   for (int q = max(0, q_end - R); q < q_end; ++q) mbar_wait(full + q % R, (q / R) & 1, max_spins);
 }
 
+constexpr int kWbCols = 2;  // columns a thread writes back at a time
+
+// The upper supernodes' columns, by the CTAs of the block kernels as they run
+// out of blocks (in a launch of its own the solve of the 500 x 500 cloth took
+// 0.241 ms instead of 0.235 in FP64, 0.185 instead of 0.174 in FP32; by the
+// producer warps during their first block 0.246 and 0.196): the backward kernel writes them
+// back as it does its blocks' and clears their y for the next solve, whose
+// forward kernel clears their x (the backward kernel still reads it).  Two columns
+// a thread and pass, every load of the pass before its stores.
+// (Not inlined: the block kernel's loops keep their registers.)
+template <typename T>
+__device__ __noinline__ void write_back_upper(const int* __restrict__ cols, int n_cols, const int* __restrict__ perm,
+                                              const T* x, T* y, int n, double* __restrict__ v, double* __restrict__ qk,
+                                              const double* __restrict__ q, double dt, int mode) {
+  const int step = gridDim.x * blockDim.x;
+  for (int k0 = blockIdx.x * blockDim.x + threadIdx.x; k0 < n_cols; k0 += kWbCols * step) {
+    int col[kWbCols];
+    int64_t vtx[kWbCols];
+    double val[kWbCols][3], qv[kWbCols][3];
+#pragma unroll
+    for (int j = 0; j < kWbCols; ++j) col[j] = k0 + j * step < n_cols ? cols[k0 + j * step] : -1;
+#pragma unroll
+    for (int j = 0; j < kWbCols; ++j) vtx[j] = col[j] >= 0 ? perm[col[j]] : -1;
+#pragma unroll
+    for (int j = 0; j < kWbCols; ++j)
+      if (col[j] >= 0)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          val[j][c] = (double)ldcg(x + col[j] + (int64_t)c * n);
+          qv[j][c] = q[3 * vtx[j] + c];
+          if (mode == 1) val[j][c] += v[3 * vtx[j] + c];
+        }
+#pragma unroll
+    for (int j = 0; j < kWbCols; ++j)
+      if (col[j] >= 0)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          y[col[j] + (int64_t)c * n] = T(0);
+          v[3 * vtx[j] + c] = val[j][c];
+          qk[3 * vtx[j] + c] = qv[j][c] + dt * val[j][c];
+        }
+  }
+}
+template <typename T>
+__device__ __forceinline__ void clear_upper(const DPlan& P, T* x, int n) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < P.n_upper; k += gridDim.x * blockDim.x) {
+    const int64_t col = P.upper_cols[k];
+    x[col] = x[col + n] = x[col + 2 * (int64_t)n] = T(0);
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kBlockMaxThreads, 1) k_block_forward(DPlan P, const T* __restrict__ W, T* b, T* y,
-                                                                    int n, SweepSync sy) {
+                                                                    T* x, int n, SweepSync sy) {
   trace_stamp(sy.trace, DTrace::kSolve);
   griddep_launch_dependents();  // the first upper level may start on SMs this sweep leaves
   constexpr int KE = kSlabElems;
@@ -354,6 +405,7 @@ __global__ void __launch_bounds__(kBlockMaxThreads, 1) k_block_forward(DPlan P, 
   if (threadIdx.x == 0) {
     s_ticket = atomicAdd(sy.queue + 2, 1);
     s_failed = 0;
+    if (blockIdx.x == 0) sy.queue[3] = 0;  // the last solve's backward tickets
   }
   __syncthreads();
   for (;;) {
@@ -473,6 +525,7 @@ __global__ void __launch_bounds__(kBlockMaxThreads, 1) k_block_forward(DPlan P, 
   // a wait gave up somewhere: every copy the producer issued lands before
   // the CTA exits
   if (s_failed && producer && lane == 0) drain_ring(sm.full, q_issued, R, sy.max_spins);
+  clear_upper(P, x, n);
 }
 
 // v[perm[k]] = x_k (mode 0) or += x_k (mode 1) and q^k = q_n + dt v for the
@@ -480,7 +533,6 @@ __global__ void __launch_bounds__(kBlockMaxThreads, 1) k_block_forward(DPlan P, 
 // thread takes kWbCols columns a pass and issues every load of the pass
 // before its stores, so that a pass costs two dependent memory round trips
 // (the permutation, then the vertex gathers) instead of several per column.
-constexpr int kWbCols = 2;
 constexpr int kExtBatch = 4;  // ext rows per thread whose indices are loaded together
 template <typename T>
 __device__ __forceinline__ void write_back_columns(const T* sv, int ld, int nc, const int* __restrict__ perm,
@@ -520,8 +572,8 @@ __device__ __forceinline__ void write_back_columns(const T* sv, int ld, int nc, 
 
 template <typename T>
 __global__ void __launch_bounds__(kBlockMaxThreads, 1) k_block_backward(DPlan P, const T* __restrict__ W,
-                                                                     const T* __restrict__ y, const T* x, int n,
-                                                                     SweepSync sy, WriteBack wb) {
+                                                                     T* y, const T* x, int n, SweepSync sy,
+                                                                     WriteBack wb) {
   griddep_launch_dependents();
   constexpr int KE = kSlabElems;
   const int R = P.ring_b;
@@ -689,6 +741,10 @@ __global__ void __launch_bounds__(kBlockMaxThreads, 1) k_block_backward(DPlan P,
   }
   if (s_failed && producer && lane == 0) drain_ring(sm.full, q_issued, R, sy.max_spins);
   griddep_wait();  // a CTA without a block completes after the launch before it too
+  write_back_upper(P.upper_cols, P.n_upper, P.perm, x, y, n, wb.v, wb.qk, wb.q, wb.dt, wb.mode);
+  // the queues of the launches before this one, and the solve counter
+  if (blockIdx.x == 0 && threadIdx.x < 3) sy.queue[threadIdx.x] = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *sy.epoch += 1ULL;
 }
 
 // ---------------------------------------------------------- upper items
@@ -1004,43 +1060,6 @@ __global__ void __launch_bounds__(32 * kLevelWarps)
   if (!waited) griddep_wait();
 }
 
-// After the backward sweep, for the upper supernodes' columns: v[perm] = x
-// (mode 0) or v[perm] += x (mode 1), q^k = q_n + dt v, and x, y cleared for
-// the next solve (the blocks' columns are written back by the backward sweep
-// and their y is overwritten by the next forward sweep); one thread rewinds
-// the work queues and advances the solve counter.
-template <typename T>
-__global__ void k_solve_post(DPlan P, T* __restrict__ x, T* __restrict__ y, int n, WriteBack wb, SweepSync sy) {
-  griddep_wait();  // launched as a programmatic dependent of the block backward sweep
-  double* __restrict__ v = wb.v;
-  double* __restrict__ qk = wb.qk;
-  const double* __restrict__ q = wb.q;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < P.n_upper; k += gridDim.x * blockDim.x) {
-    const int col = P.upper_cols[k];
-    const int64_t vtx = P.perm[col];
-    // every load before the first store (the arrays do not alias)
-    double val[3], qv[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      val[c] = (double)x[col + (int64_t)c * n];
-      qv[c] = q[3 * vtx + c];
-    }
-    if (wb.mode == 1)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) val[c] += v[3 * vtx + c];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const int64_t o = col + (int64_t)c * n;
-      x[o] = 0;
-      y[o] = 0;
-      v[3 * vtx + c] = val[c];
-      qk[3 * vtx + c] = qv[c] + wb.dt * val[c];
-    }
-  }
-  if (blockIdx.x == 0 && threadIdx.x < 4) sy.queue[threadIdx.x] = 0;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *sy.epoch += 1ULL;
-}
-
 // Clears the solve vectors and rewinds the queues (first use / timing runs).
 template <typename T>
 __global__ void k_solve_prep(int n, T* x, T* y, SweepSync sy) {
@@ -1138,8 +1157,8 @@ bool configure_solve(DPlan& P, int shape) {
 template <typename T>
 void launch_solve_sweeps(cudaStream_t st, const DPlan& P, const T* Wf, const T* Wb, T* b, T* y, T* x, int n,
                          SweepSync sy, WriteBack wb, cudaEvent_t* marks) {
-  // marks (optional): 4 events recorded between the five launches
-  k_block_forward<T><<<P.grid_bf, 32 * (P.block_warps + 1), P.smem_f, st>>>(P, Wf, b, y, n, sy);
+  // marks (optional): 4 events recorded after the four parts
+  k_block_forward<T><<<P.grid_bf, 32 * (P.block_warps + 1), P.smem_f, st>>>(P, Wf, b, y, x, n, sy);
   if (marks) cudaEventRecord(marks[0], st);
   auto level = [&](bool fwd, int lo, int hi) {
     const int grid = std::max(1, std::min(fwd ? P.grid_lf : P.grid_lb, (hi - lo + kLevelWarps - 1) / kLevelWarps));
@@ -1158,11 +1177,9 @@ void launch_solve_sweeps(cudaStream_t st, const DPlan& P, const T* Wf, const T* 
     k_upper_backward<T><<<P.grid_ub, kSweepThreads, 0, st>>>(P, Wb, y, x, n, sy);
   }
   if (marks) cudaEventRecord(marks[2], st);
-  launch_dependent(k_block_backward<T>, P.grid_bb, 32 * (P.block_warps + 1), (size_t)P.smem_b, st, P, Wb,
-                   static_cast<const T*>(y), static_cast<const T*>(x), n, sy, wb);
+  launch_dependent(k_block_backward<T>, P.grid_bb, 32 * (P.block_warps + 1), (size_t)P.smem_b, st, P, Wb, y,
+                   static_cast<const T*>(x), n, sy, wb);
   if (marks) cudaEventRecord(marks[3], st);
-  launch_dependent(k_solve_post<T>, std::max(1, std::min(148 * 4, (P.n_upper + 255) / 256)), 256, 0, st, P, x, y, n,
-                   wb, sy);
 }
 template <typename T>
 void launch_solve_prep(cudaStream_t st, int n, T* x, T* y, SweepSync sy) {
