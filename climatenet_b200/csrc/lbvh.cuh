@@ -75,7 +75,7 @@ __device__ __forceinline__ unsigned int spread10(unsigned int v) {
   return v;
 }
 
-// Leaf boxes and Morton keys (key = morton << 32 | triangle, unique).
+// Leaf boxes (where tlo is given) and Morton keys (key = morton << 32 | triangle, unique).
 __global__ void k_tri_keys(int nt, const double* __restrict__ q, const int* __restrict__ tris, int v0,
                            const unsigned long long* __restrict__ bbox, double* tlo, double* thi,
                            unsigned long long* key, int* val) {
@@ -84,8 +84,10 @@ __global__ void k_tri_keys(int nt, const double* __restrict__ q, const int* __re
   const double3 a = ld3(q, tris[3 * t]), b = ld3(q, tris[3 * t + 1]), c = ld3(q, tris[3 * t + 2]);
   double3 lo, hi;
   tri_box(a, b, c, &lo, &hi);
-  st3(tlo, t, lo);
-  st3(thi, t, hi);
+  if (tlo) {
+    st3(tlo, t, lo);
+    st3(thi, t, hi);
+  }
   (void)v0;
   const double bl[3] = {from_ord(bbox[0]), from_ord(bbox[1]), from_ord(bbox[2])};
   const double bh[3] = {from_ord(bbox[3]), from_ord(bbox[4]), from_ord(bbox[5])};

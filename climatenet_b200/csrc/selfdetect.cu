@@ -52,14 +52,12 @@ constexpr int kPairSpins = 1 << 22;  // polls before a wait of the pairing gives
 
 struct SelfWS {
   int max_nt = 0, max_nv = 0, hit_cap = 0;
-  double *tlo = nullptr, *thi = nullptr;             // 3 nt leaf boxes (triangle order)
   unsigned long long *mkey = nullptr, *mkey2 = nullptr;
   int *mval = nullptr, *mval2 = nullptr;             // sorted leaf -> triangle
   int *left = nullptr, *right = nullptr, *parent = nullptr, *leaf_parent = nullptr;
-  double *nlo = nullptr, *nhi = nullptr;             // 3 (nt-1) node boxes
   int* visits = nullptr;
   unsigned long long* bbox = nullptr;                // 6 ordered-bit min/max
-  int* n_hits = nullptr;
+  int* n_hits = nullptr;  // two words: the count, and err
   unsigned long long *hkey = nullptr, *hkey2 = nullptr;
   int *hval = nullptr, *hval2 = nullptr;
   double* hbary = nullptr;
@@ -98,52 +96,167 @@ T* salloc(size_t n) {
   return p;
 }
 
-__device__ __forceinline__ void child_box(int c, const int* mval, const double* tlo, const double* thi,
-                                          const double* nlo, const double* nhi, double3* lo, double3* hi) {
-  if (c < 0) {
-    const int t = mval[~c];
-    *lo = make_double3(__ldcg(tlo + 3 * t), __ldcg(tlo + 3 * t + 1), __ldcg(tlo + 3 * t + 2));
-    *hi = make_double3(__ldcg(thi + 3 * t), __ldcg(thi + 3 * t + 1), __ldcg(thi + 3 * t + 2));
+// Traversal: kWalkLanes lanes walk the hierarchy for one vertex.  Both children of a
+// node are tested at their parent (one node record), the overlapping internal
+// children go to the group's stack in shared memory, from which the lanes take
+// up to kWalkLanes nodes at a time; overlapping leaf children are candidates.  The set
+// found does not depend on the order.
+//
+// A walk is a chain of node loads (some 60 to 100 of them with one lane a
+// vertex) and bound by their latency until the chip is full of walks; then the
+// lanes that find no node cost more than the shorter chains save.  Measured (ncu):
+// 14k vertices, kPairsOnly, 37 us (4 lanes 68, 16 lanes 44, one lane and an atomic
+// a pair 197); 49k vertices, kStep, 99 us (4 lanes 116, 16 lanes 109, one lane
+// 146); 131k and 250k vertices: one lane 217 and 256 us, two lanes 397 at 131k.
+// So the step's meshes above kWalkVertices keep one lane (k_traverse_slots).  A
+// stack that grows past kWalkWide is walked depth first, one node at a time, which
+// bounds it by the tree's depth.
+//
+// Mode kStep: candidates that do not contain the vertex go to the vertex's
+// kHitSlots slots, their number to hcount.  Mode kPairsOnly: every candidate
+// (v, t) goes to hkey, a vertex's together and in triangle order unless it has
+// more than some 50 (then kWalkUnsorted is set in *err).  Mode kHits: candidates
+// that survive the closest-point filter and can pair go to hkey / hval / hbary.
+constexpr int kTraverseThreads = 128, kWalkLanes = 8, kWalkWide = 32, kWalkDepth = 64, kWalkBuf = 64;
+constexpr int kWalkVertices = 65536;
+constexpr int kWalkOverflow = 2, kWalkUnsorted = 4;  // bits of *err (kPairsOnly, kHits)
+enum WalkMode { kStep, kPairsOnly, kHits };
+constexpr int kWalkStack = kWalkWide + 2 * kWalkLanes + kWalkDepth;
+template <int kMode>
+__global__ void __launch_bounds__(kTraverseThreads)
+    k_traverse(int nv, int nt, const double* __restrict__ q, const int* __restrict__ tris, int v0, double tol,
+               const WNode* __restrict__ nodes, int* __restrict__ hcount, int* __restrict__ slot_tri, int* n_hits,
+               int cap, unsigned long long* hkey, int* hval, double* hbary, int* err) {
+  constexpr int G = kWalkLanes, kGroups = kTraverseThreads / G, kStack = kWalkStack, kBuf = kWalkBuf;
+  __shared__ int stacks[kGroups * kStack];
+  __shared__ int bufs[kMode == kStep ? 1 : kGroups * kBuf];
+  const int lane = threadIdx.x & 31, gl = lane % G, group = threadIdx.x / G;
+  const unsigned int mask = ((1u << G) - 1u) << (lane - gl), below = mask & ((1u << lane) - 1u);
+  const int v = blockIdx.x * kGroups + group;
+  if (v >= nv) return;
+  int* st = stacks + group * kStack;
+  int* buf = bufs + (kMode == kStep ? 0 : group * kBuf);
+  const double t = 1.1 * tol;
+  const double3 x = ld3(q, v0 + v);
+  const int gv = v0 + v;
+  int* slots = slot_tri + (int64_t)v * kHitSlots;
+  int count = 0, flushes = 0;
+  auto own = [&](int tri) {
+    return __ldg(tris + 3 * tri) == gv || __ldg(tris + 3 * tri + 1) == gv || __ldg(tris + 3 * tri + 2) == gv;
+  };
+  // the buffered candidates out (kPairsOnly, kHits)
+  auto flush = [&]() {
+    __syncwarp(mask);
+    if (kMode == kPairsOnly && count > 0) {
+      int base = 0;
+      if (gl == 0) {
+        base = atomicAdd(n_hits, count);
+        if (++flushes > 1) atomicOr(err, kWalkUnsorted);
+      }
+      base = __shfl_sync(mask, base, lane - gl);
+      for (int i = gl; i < count; i += G) {
+        const int tri = buf[i];
+        int rank = 0;
+        for (int j = 0; j < count; ++j) rank += buf[j] < tri;
+        if (base + rank < cap) hkey[base + rank] = ((unsigned long long)v << 32) | (unsigned int)tri;
+      }
+    } else if (kMode == kHits) {
+      for (int i = gl; i < count; i += G) {
+        const int tri = buf[i];
+        double3 cp, w;
+        closest_point(x, ld3(q, tris[3 * tri]), ld3(q, tris[3 * tri + 1]), ld3(q, tris[3 * tri + 2]), tol, &cp, &w);
+        const double3 dd = cp - x;
+        if (!(dot3(dd, dd) < tol * tol)) continue;
+        if (w.x == 0 || w.y == 0 || w.z == 0) continue;
+        const int k = atomicAdd(n_hits, 1);
+        if (k < cap) {
+          hkey[k] = ((unsigned long long)v << 32) | (unsigned int)tri;
+          hval[k] = k;
+          st3(hbary, k, w);
+        }
+      }
+    }
+    __syncwarp(mask);
+    count = 0;
+  };
+  // a lane's candidate (hit false: none) into the group's list
+  auto add = [&](bool hit, int tri) {
+    if (kMode != kPairsOnly && hit) hit = !own(tri);
+    const unsigned int m = __ballot_sync(mask, hit);
+    const int at = count + __popc(m & below);
+    if (hit) {
+      if (kMode == kStep) {
+        if (at < kHitSlots) slots[at] = tri;
+      } else {
+        buf[at] = tri;
+      }
+    }
+    count += __popc(m);
+  };
+  if (nt == 1) {
+    double3 tl, th;
+    tri_box(ld3(q, tris[0]), ld3(q, tris[1]), ld3(q, tris[2]), &tl, &th);
+    add(gl == 0 && box_overlap(x, t, tl, th), 0);
   } else {
-    *lo = make_double3(__ldcg(nlo + 3 * c), __ldcg(nlo + 3 * c + 1), __ldcg(nlo + 3 * c + 2));
-    *hi = make_double3(__ldcg(nhi + 3 * c), __ldcg(nhi + 3 * c + 1), __ldcg(nhi + 3 * c + 2));
+    int sp = 1;
+    if (gl == 0) st[0] = 0;
+    __syncwarp(mask);
+    while (sp > 0) {
+      const int take = sp > kWalkWide ? 1 : min(sp, G);
+      const int node = gl < take ? st[sp - 1 - gl] : -1;
+      sp -= take;
+      __syncwarp(mask);
+      bool o0 = false, o1 = false;
+      int c0 = 0, c1 = 0;
+      if (node >= 0) {
+        // the 112-byte record in seven 16-byte loads
+        const double2* r = reinterpret_cast<const double2*>(nodes + node);
+        const double2 b01 = __ldg(r), b23 = __ldg(r + 1), b45 = __ldg(r + 2), b67 = __ldg(r + 3),
+                      b89 = __ldg(r + 4), b1011 = __ldg(r + 5);
+        const int4 chv = __ldg(reinterpret_cast<const int4*>(r + 6));
+        c0 = chv.x;
+        c1 = chv.y;
+        o0 = box_overlap(x, t, make_double3(b01.x, b01.y, b23.x), make_double3(b23.y, b45.x, b45.y));
+        o1 = box_overlap(x, t, make_double3(b67.x, b67.y, b89.x), make_double3(b89.y, b1011.x, b1011.y));
+      }
+      const bool p0 = o0 && c0 >= 0, p1 = o1 && c1 >= 0;
+      const unsigned int m0 = __ballot_sync(mask, p0), m1 = __ballot_sync(mask, p1);
+      const int n0 = __popc(m0), n1 = __popc(m1);
+      if (sp + n0 + n1 > kStack) {
+        if (gl == 0) atomicOr(err, kMode == kStep ? kErrSelfStack : kWalkOverflow);
+        break;
+      }
+      if (p0) st[sp + __popc(m0 & below)] = c0;
+      if (p1) st[sp + n0 + __popc(m1 & below)] = c1;
+      sp += n0 + n1;
+      const bool any_leaf = __any_sync(mask, (o0 && c0 < 0) || (o1 && c1 < 0));
+      if (any_leaf) {
+        if (kMode != kStep && count + 2 * G > kBuf) flush();
+        add(o0 && c0 < 0, ~c0);
+        add(o1 && c1 < 0, ~c1);
+      }
+      __syncwarp(mask);
+    }
+  }
+  if (kMode != kStep) {
+    flush();
+  } else if (gl == 0) {
+    if (count > kHitSlots) {
+      atomicOr(err, kErrSelfHits);
+      count = kHitSlots;
+    }
+    hcount[v] = count;
   }
 }
 
-// Bottom-up refit: the second child to arrive computes the parent's box.
-__global__ void k_refit(int n, const int* __restrict__ mval, const double* tlo, const double* thi, const int* left,
-                        const int* right, const int* parent, const int* leaf_parent, double* nlo, double* nhi,
-                        int* visits) {
-  const int leaf = blockIdx.x * blockDim.x + threadIdx.x;
-  if (leaf >= n) return;
-  int p = leaf_parent[leaf];
-  while (p >= 0) {
-    __threadfence();
-    if (atomicAdd(visits + p, 1) == 0) return;
-    __threadfence();
-    double3 l0, h0, l1, h1;
-    child_box(left[p], mval, tlo, thi, nlo, nhi, &l0, &h0);
-    child_box(right[p], mval, tlo, thi, nlo, nhi, &l1, &h1);
-    const double3 lo = make_double3(fmin(l0.x, l1.x), fmin(l0.y, l1.y), fmin(l0.z, l1.z));
-    const double3 hi = make_double3(fmax(h0.x, h1.x), fmax(h0.y, h1.y), fmax(h0.z, h1.z));
-    __stcg(nlo + 3 * p, lo.x);
-    __stcg(nlo + 3 * p + 1, lo.y);
-    __stcg(nlo + 3 * p + 2, lo.z);
-    __stcg(nhi + 3 * p, hi.x);
-    __stcg(nhi + 3 * p + 1, hi.y);
-    __stcg(nhi + 3 * p + 2, hi.z);
-    p = parent[p];
-  }
-}
-
-// Step-path traversal: both children are tested at their parent (one node
+// Step-path traversal of large meshes, one lane a vertex: both children are tested at their parent (one node
 // record load), overlapping leaf children are handled on the spot, the walk
 // continues into the first overlapping internal child and keeps the other on
 // a per-thread stack in shared memory (column-major: no bank conflicts).  A
 // candidate is a triangle whose box overlaps the vertex's query box and that
 // does not contain the vertex; candidates go to the vertex's slots,
 // unordered, and the closest-point filter runs in k_filter_candidates.
-constexpr int kTraverseThreads = 128, kTraverseStack = 48;
+constexpr int kTraverseStack = 48;
 __global__ void __launch_bounds__(kTraverseThreads)
     k_traverse_slots(int nv, int nt, const double* __restrict__ q, const int* __restrict__ tris, int v0, double tol,
                      const WNode* __restrict__ nodes, int* __restrict__ hcount, int* __restrict__ slot_tri,
@@ -202,6 +315,12 @@ __global__ void __launch_bounds__(kTraverseThreads)
     count = kHitSlots;
   }
   hcount[v] = count;
+}
+
+template <int kMode, typename... Args>
+void launch_traverse(cudaStream_t st, int nv, Args... args) {
+  constexpr int per = kTraverseThreads / kWalkLanes;
+  k_traverse<kMode><<<(nv + per - 1) / per, kTraverseThreads, 0, st>>>(nv, args...);
 }
 
 // The closest-point filter and the pairing precondition of mode 1 below on
@@ -265,61 +384,6 @@ __global__ void k_compact_hits(int nv, const double* __restrict__ q, const int* 
     hkey[h] = ((unsigned long long)v << 32) | (unsigned int)tri;
     hval[h] = h;
     st3(hbary, h, w);
-  }
-}
-
-// Per-vertex traversal.  mode 0: emit every box candidate (v, t);
-// mode 1: emit hits that survive the closest-point filter and can pair.
-__global__ void k_traverse(int nv, int nt, const double* __restrict__ q, const int* __restrict__ tris, int v0,
-                           double tol, const int* __restrict__ mval, const double* __restrict__ tlo,
-                           const double* __restrict__ thi, const int* __restrict__ left, const int* __restrict__ right,
-                           const double* __restrict__ nlo, const double* __restrict__ nhi, int mode, int* n_hits,
-                           int cap, unsigned long long* hkey, int* hval, double* hbary, int* err) {
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nv) return;
-  const double t = 1.1 * tol;
-  const double tol_sq = tol * tol;
-  const double3 x = ld3(q, v0 + v);
-  int stack[64];
-  int sp = 0;
-  stack[sp++] = (nt == 1) ? ~0 : 0;
-  while (sp > 0) {
-    const int node = stack[--sp];
-    if (node < 0) {
-      const int tri = mval[~node];
-      const double3 lo = ld3(tlo, tri), hi = ld3(thi, tri);
-      if (!box_overlap(x, t, lo, hi)) continue;
-      if (mode == 0) {
-        const int k = atomicAdd(n_hits, 1);
-        if (k < cap) {
-          hkey[k] = ((unsigned long long)v << 32) | (unsigned int)tri;
-          hval[k] = k;
-        }
-        continue;
-      }
-      const int ia = tris[3 * tri] - v0, ib = tris[3 * tri + 1] - v0, ic = tris[3 * tri + 2] - v0;
-      if (ia == v || ib == v || ic == v) continue;
-      double3 cp, w;
-      closest_point(x, ld3(q, v0 + ia), ld3(q, v0 + ib), ld3(q, v0 + ic), tol, &cp, &w);
-      const double3 dd = cp - x;
-      if (!(dot3(dd, dd) < tol_sq)) continue;
-      if (w.x == 0 || w.y == 0 || w.z == 0) continue;
-      const int k = atomicAdd(n_hits, 1);
-      if (k < cap) {
-        hkey[k] = ((unsigned long long)v << 32) | (unsigned int)tri;
-        hval[k] = k;
-        st3(hbary, k, w);
-      }
-      continue;
-    }
-    const double3 lo = ld3(nlo, node), hi = ld3(nhi, node);
-    if (!box_overlap(x, t, lo, hi)) continue;
-    if (sp + 2 > 64) {
-      atomicExch(err, 2);
-      return;
-    }
-    stack[sp++] = left[node];
-    stack[sp++] = right[node];
   }
 }
 
@@ -822,8 +886,6 @@ void ws_alloc(SelfWS& w, int nv, int nt, int hit_cap, int slot_cap) {
   w.max_nv = nv;
   w.max_nt = nt;
   w.hit_cap = hit_cap;
-  w.tlo = salloc<double>(3 * (size_t)nt);
-  w.thi = salloc<double>(3 * (size_t)nt);
   w.mkey = salloc<unsigned long long>(nt);
   w.mkey2 = salloc<unsigned long long>(nt);
   w.mval = salloc<int>(nt);
@@ -832,17 +894,15 @@ void ws_alloc(SelfWS& w, int nv, int nt, int hit_cap, int slot_cap) {
   w.right = salloc<int>(nt);
   w.parent = salloc<int>(nt);
   w.leaf_parent = salloc<int>(nt);
-  w.nlo = salloc<double>(3 * (size_t)nt);
-  w.nhi = salloc<double>(3 * (size_t)nt);
   w.visits = salloc<int>(nt);
   w.bbox = salloc<unsigned long long>(6);
-  w.n_hits = salloc<int>(1);
+  w.n_hits = salloc<int>(2);
+  w.err = w.n_hits + 1;
   w.hkey = salloc<unsigned long long>(hit_cap);
   w.hkey2 = salloc<unsigned long long>(hit_cap);
   w.hval = salloc<int>(hit_cap);
   w.hval2 = salloc<int>(hit_cap);
   w.hbary = salloc<double>(3 * (size_t)hit_cap);
-  w.err = salloc<int>(1);
   w.hcount = salloc<int>(nv);
   w.hoff = salloc<int>(nv);
   w.slot_tri = salloc<int>((size_t)nv * kHitSlots);
@@ -857,9 +917,9 @@ void ws_alloc(SelfWS& w, int nv, int nt, int hit_cap, int slot_cap) {
 }
 
 void ws_free(SelfWS& w) {
-  void* ptrs[] = {w.tlo, w.thi, w.mkey, w.mkey2, w.mval, w.mval2, w.left, w.right, w.parent, w.leaf_parent,
-                  w.nlo, w.nhi, w.visits, w.bbox, w.n_hits, w.hkey, w.hkey2, w.hval, w.hval2, w.hbary,
-                  w.reg, w.reg_n, w.touched, w.n_touched, w.err, w.deg, w.uf, w.dist, w.seed, w.cobst, w.cdeg1,
+  void* ptrs[] = {w.mkey, w.mkey2, w.mval, w.mval2, w.left, w.right, w.parent, w.leaf_parent,
+                  w.visits, w.bbox, w.n_hits, w.hkey, w.hkey2, w.hval, w.hval2, w.hbary,
+                  w.reg, w.reg_n, w.touched, w.n_touched, w.deg, w.uf, w.dist, w.seed, w.cobst, w.cdeg1,
                   w.cmin, w.elev, w.lcount, w.cub_tmp, w.wnodes, w.hcount, w.hoff, w.slot_tri, w.n_total,
                   w.s_mval, w.s_left, w.s_right, w.s_parent, w.s_leaf_parent, w.s_visits,
                   w.pair_done, w.paired, w.pair_hit, w.pair_base, w.pair_ticket};
@@ -868,37 +928,59 @@ void ws_free(SelfWS& w) {
   w = SelfWS{};
 }
 
+// Bits that hold the values 0 .. n - 1.
+int bits_for(int n) {
+  int b = 1;
+  while (b < 31 && (1 << b) < n) ++b;
+  return b;
+}
+
 // Builds the LBVH over triangles [t0, t0+nt) (scene-global vertex indices
 // with vertices [v0, v0+nv)) and traverses it from every vertex of the range.
-// Returns the number of emitted records (may exceed the capacity).
-int detect_mesh(SelfWS& w, const double* q, const int* tris_global, int v0, int nv, int nt, double tol, int mode,
+// Returns the number of emitted records (may exceed the capacity); up to it they
+// are in hkey2 (kHits: with hval2 their places in hbary) sorted by (vertex, triangle).
+template <int kMode>
+int detect_mesh(SelfWS& w, const double* q, const int* tris_global, int v0, int nv, int nt, double tol,
                 cudaStream_t st) {
   const int tb = 256;
-  const unsigned long long init[6] = {~0ULL, ~0ULL, ~0ULL, 0ULL, 0ULL, 0ULL};
-  CKS(cudaMemcpyAsync(w.bbox, init, sizeof(init), cudaMemcpyHostToDevice, st));
-  k_bbox<<<std::min(1024, (nv + tb - 1) / tb), tb, 0, st>>>(nv, q + 3 * (size_t)v0, w.bbox);
-  k_tri_keys<<<(nt + tb - 1) / tb, tb, 0, st>>>(nt, q, tris_global, v0, w.bbox, w.tlo, w.thi, w.mkey, w.mval);
   size_t bytes = w.cub_bytes;
-  CKS(cub::DeviceRadixSort::SortPairs(w.cub_tmp, bytes, w.mkey, w.mkey2, w.mval, w.mval2, nt, 0, 64, st));
   if (nt > 1) {
+    const unsigned long long init[6] = {~0ULL, ~0ULL, ~0ULL, 0ULL, 0ULL, 0ULL};
+    CKS(cudaMemcpyAsync(w.bbox, init, sizeof(init), cudaMemcpyHostToDevice, st));
+    k_bbox<<<std::min(1024, (nv + tb - 1) / tb), tb, 0, st>>>(nv, q + 3 * (size_t)v0, w.bbox);
+    k_tri_keys<<<(nt + tb - 1) / tb, tb, 0, st>>>(nt, q, tris_global, v0, w.bbox, nullptr, nullptr, w.mkey, w.mval);
+    // the keys come in triangle order and the sort is stable: the Morton bits
+    // give the order of the whole key
+    CKS(cub::DeviceRadixSort::SortPairs(w.cub_tmp, bytes, w.mkey, w.mkey2, w.mval, w.mval2, nt, 32, 62, st));
     k_build<<<(nt - 1 + tb - 1) / tb, tb, 0, st>>>(nt, w.mkey2, w.left, w.right, w.parent, w.leaf_parent);
     CKS(cudaMemsetAsync(w.visits, 0, sizeof(int) * nt, st));
-    k_refit<<<(nt + tb - 1) / tb, tb, 0, st>>>(nt, w.mval2, w.tlo, w.thi, w.left, w.right, w.parent, w.leaf_parent,
-                                               w.nlo, w.nhi, w.visits);
+    k_refit_wide<<<(nt + tb - 1) / tb, tb, 0, st>>>(nt, w.mval2, q, tris_global, w.left, w.parent, w.leaf_parent,
+                                                    w.wnodes, w.visits);
   }
-  CKS(cudaMemsetAsync(w.n_hits, 0, sizeof(int), st));
-  CKS(cudaMemsetAsync(w.err, 0, sizeof(int), st));
-  k_traverse<<<(nv + tb - 1) / tb, tb, 0, st>>>(nv, nt, q, tris_global, v0, tol, w.mval2, w.tlo, w.thi, w.left,
-                                               w.right, w.nlo, w.nhi, mode, w.n_hits, w.hit_cap, w.hkey, w.hval,
-                                               w.hbary, w.err);
-  int nh = 0, err = 0;
-  CKS(cudaMemcpyAsync(&nh, w.n_hits, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CKS(cudaMemcpyAsync(&err, w.err, sizeof(int), cudaMemcpyDeviceToHost, st));
+  // the count and the error bits lie side by side: one clear, one read
+  CKS(cudaMemsetAsync(w.n_hits, 0, 2 * sizeof(int), st));
+  launch_traverse<kMode>(st, nv, nt, q, tris_global, v0, tol, w.wnodes, (int*)nullptr, (int*)nullptr, w.n_hits,
+                         w.hit_cap, w.hkey, w.hval, w.hbary, w.err);
+  int res[2] = {0, 0};
+  CKS(cudaMemcpyAsync(res, w.n_hits, sizeof(res), cudaMemcpyDeviceToHost, st));
   CKS(cudaStreamSynchronize(st));
-  if (err) throw std::overflow_error("BVH traversal stack overflow (a vertex's walk needs more than the stack holds)");
+  const int nh = res[0], err = res[1];
+  if (err & kWalkOverflow)
+    throw std::overflow_error("BVH traversal stack overflow (a vertex's walk needs more than the stack holds)");
   if (nh > 0 && nh <= w.hit_cap) {
-    int bits = 64;
-    CKS(cub::DeviceRadixSort::SortPairs(w.cub_tmp, bytes, w.hkey, w.hkey2, w.hval, w.hval2, nh, 0, bits, st));
+    const int tbits = bits_for(nt), vbits = bits_for(nv);
+    if (kMode == kHits) {
+      CKS(cub::DeviceRadixSort::SortPairs(w.cub_tmp, bytes, w.hkey, w.hkey2, w.hval, w.hval2, nh, 0, tbits, st));
+      std::swap(w.hkey, w.hkey2);
+      std::swap(w.hval, w.hval2);
+      CKS(cub::DeviceRadixSort::SortPairs(w.cub_tmp, bytes, w.hkey, w.hkey2, w.hval, w.hval2, nh, 32, 32 + vbits, st));
+    } else {
+      if (err & kWalkUnsorted) {
+        CKS(cub::DeviceRadixSort::SortKeys(w.cub_tmp, bytes, w.hkey, w.hkey2, nh, 0, tbits, st));
+        std::swap(w.hkey, w.hkey2);
+      }
+      CKS(cub::DeviceRadixSort::SortKeys(w.cub_tmp, bytes, w.hkey, w.hkey2, nh, 32, 32 + vbits, st));
+    }
   }
   return nh;
 }
@@ -918,7 +1000,7 @@ void detect_mesh_step(SelfWS& w, const double* q, const int* tris_global, int v0
     const unsigned long long init[6] = {~0ULL, ~0ULL, ~0ULL, 0ULL, 0ULL, 0ULL};
     CKS(cudaMemcpyAsync(w.bbox, init, sizeof(init), cudaMemcpyHostToDevice, st));
     k_bbox<<<std::min(1024, (nv + tb - 1) / tb), tb, 0, st>>>(nv, q + 3 * (size_t)v0, w.bbox);
-    k_tri_keys<<<(nt + tb - 1) / tb, tb, 0, st>>>(nt, q, tris_global, v0, w.bbox, w.tlo, w.thi, w.mkey, w.mval);
+    k_tri_keys<<<(nt + tb - 1) / tb, tb, 0, st>>>(nt, q, tris_global, v0, w.bbox, nullptr, nullptr, w.mkey, w.mval);
     // key = morton << 32 | triangle and the sort is stable on triangles in
     // ascending order: the 30 Morton bits give the full key order
     size_t bytes = w.cub_bytes;
@@ -931,8 +1013,12 @@ void detect_mesh_step(SelfWS& w, const double* q, const int* tris_global, int v0
     k_refit_wide<<<(nt + tb - 1) / tb, tb, 0, st>>>(nt, mval, q, tris_global, left, parent, leaf_parent, nodes,
                                                     w.s_visits + t0);
   }
-  k_traverse_slots<<<(nv + kTraverseThreads - 1) / kTraverseThreads, kTraverseThreads, 0, st>>>(
-      nv, nt, q, tris_global, v0, tol, nodes, w.hcount, w.slot_tri, err_word);
+  if (nv <= kWalkVertices)
+    launch_traverse<kStep>(st, nv, nt, q, tris_global, v0, tol, nodes, w.hcount, w.slot_tri, (int*)nullptr, 0,
+                           (unsigned long long*)nullptr, (int*)nullptr, (double*)nullptr, err_word);
+  else
+    k_traverse_slots<<<(nv + kTraverseThreads - 1) / kTraverseThreads, kTraverseThreads, 0, st>>>(
+        nv, nt, q, tris_global, v0, tol, nodes, w.hcount, w.slot_tri, err_word);
   k_filter_candidates<<<(nv + tb - 1) / tb, tb, 0, st>>>(nv, q, tris_global, v0, tol, w.hcount, w.slot_tri);
   size_t bytes = w.cub_bytes;
   CKS(cub::DeviceScan::ExclusiveSum(w.cub_tmp, bytes, w.hcount, w.hoff, nv, st));
@@ -1075,7 +1161,8 @@ int standalone_candidates(const double* pos, int nv, const int* tris, int nt, do
     CKS(cudaMemcpy(dt, tris, 3 * sizeof(int) * nt, cudaMemcpyHostToDevice));
     int hit_cap = std::max(1024, cap);
     ws_alloc(w, nv, nt, hit_cap, nv);
-    int nh = detect_mesh(w, dq, dt, 0, nv, nt, tol, 0, 0);
+    w.wnodes = salloc<WNode>(nt);
+    int nh = detect_mesh<kPairsOnly>(w, dq, dt, 0, nv, nt, tol, 0);
     if (n) *n = nh;
     if (nh > hit_cap || nh > cap) {
       err = "candidate buffer too small";
@@ -1154,8 +1241,9 @@ int standalone_self(const double* pos, int nv, const int* tris, int nt, double t
     c.self_cap = scap;
     CKS(cudaMemset(c.n_self, 0, sizeof(int)));
     ws_alloc(w, nv, nt, std::max(1024, 4 * nv), nv);
+    w.wnodes = salloc<WNode>(nt);
     ws_alloc_pairing(w, nv, 1, 1, 1, scap);
-    int nh = detect_mesh(w, dq, dt, 0, nv, nt, tol, 1, 0);
+    int nh = detect_mesh<kHits>(w, dq, dt, 0, nv, nt, tol, 0);
     if (nh > w.hit_cap) {
       err = "hit buffer too small";
       status = PDF_CAPACITY_EXCEEDED;
@@ -1229,15 +1317,13 @@ constexpr int kNoAllocMaxPairs = 262144;
 constexpr size_t kNoAllocSortBytes = size_t(8) << 20;
 constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 // byte layout of the array (each block 256-byte aligned)
-constexpr size_t kTriBytes = align256(sizeof(double) * 3 * kNoAllocMaxTriangles);      // tlo, thi, nlo, nhi
+constexpr size_t kNodeBytes = align256(sizeof(WNode) * kNoAllocMaxTriangles);  // wnodes
 constexpr size_t kTriKeyBytes = align256(sizeof(unsigned long long) * kNoAllocMaxTriangles);  // mkey, mkey2
 constexpr size_t kTriIntBytes = align256(sizeof(int) * kNoAllocMaxTriangles);  // mval, mval2, left, right, parent, leaf_parent, visits
 constexpr size_t kPairKeyBytes = align256(sizeof(unsigned long long) * kNoAllocMaxPairs);  // hkey, hkey2
-constexpr size_t kPairIntBytes = align256(sizeof(int) * kNoAllocMaxPairs);                  // hval, hval2
-constexpr size_t kPairBaryBytes = align256(sizeof(double) * 3 * kNoAllocMaxPairs);          // hbary (unused in mode 0)
-constexpr size_t kSmallBytes = 256 * 3;                                                     // bbox, n_hits, err
-constexpr size_t kNoAllocScratchBytes = 4 * kTriBytes + 2 * kTriKeyBytes + 7 * kTriIntBytes + 2 * kPairKeyBytes +
-                                        2 * kPairIntBytes + kPairBaryBytes + kSmallBytes + kNoAllocSortBytes;
+constexpr size_t kSmallBytes = 256 * 2;                                                     // bbox, n_hits and err
+constexpr size_t kNoAllocScratchBytes = kNodeBytes + 2 * kTriKeyBytes + 7 * kTriIntBytes + 2 * kPairKeyBytes +
+                                        kSmallBytes + kNoAllocSortBytes;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
@@ -1291,10 +1377,7 @@ int noalloc_candidates(const double* positions, int nv, const int* triangles, in
   w.max_nt = nt;
   w.max_nv = nv;
   w.hit_cap = kNoAllocMaxPairs;
-  w.tlo = (double*)take(kTriBytes);
-  w.thi = (double*)take(kTriBytes);
-  w.nlo = (double*)take(kTriBytes);
-  w.nhi = (double*)take(kTriBytes);
+  w.wnodes = (WNode*)take(kNodeBytes);
   w.mkey = (unsigned long long*)take(kTriKeyBytes);
   w.mkey2 = (unsigned long long*)take(kTriKeyBytes);
   w.mval = (int*)take(kTriIntBytes);
@@ -1306,15 +1389,12 @@ int noalloc_candidates(const double* positions, int nv, const int* triangles, in
   w.visits = (int*)take(kTriIntBytes);
   w.hkey = (unsigned long long*)take(kPairKeyBytes);
   w.hkey2 = (unsigned long long*)take(kPairKeyBytes);
-  w.hval = (int*)take(kPairIntBytes);
-  w.hval2 = (int*)take(kPairIntBytes);
-  w.hbary = (double*)take(kPairBaryBytes);
   w.bbox = (unsigned long long*)take(256);
   w.n_hits = (int*)take(256);
-  w.err = (int*)take(256);
+  w.err = w.n_hits + 1;
   w.cub_tmp = take(kNoAllocSortBytes);
   w.cub_bytes = kNoAllocSortBytes;
-  const int nh = detect_mesh(w, positions, triangles, 0, nv, nt, tol, 0, st);
+  const int nh = detect_mesh<kPairsOnly>(w, positions, triangles, 0, nv, nt, tol, st);
   *n_out = nh;
   if (nh > kNoAllocMaxPairs || nh > cap) {
     err = "candidate pairs exceed the output capacity or the scratch limit (" + std::to_string(kNoAllocMaxPairs) + ")";
