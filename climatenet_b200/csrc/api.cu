@@ -541,12 +541,17 @@ void create_impl(pdf_handle* h, const pdf_scene_desc* sc, const pdf_params* p) {
   h->stats.setup_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
-// Local step: bending projections + vertex right-hand side (or residual).
+// Local step: bending projections + vertex right-hand side (or residual), one launch on small scenes.
 template <typename T>
 void launch_local(pdf_handle* h, T* b, int mode) {
   DeviceBuffers& d = h->d;
   const DModel& dm = h->dm;
   cudaStream_t st = h->stream;
+  if (dm.N <= kFusedLocal) {
+    launch_local_fused<T>(st, dm, d.qk, d.v, d.cstep, std::max(h->prm.air_damping, 0.), d.c.slot_of, d.c.f, b,
+                          h->prm.time_step, mode);
+    return;
+  }
   if (dm.B > 0) k_bend_proj<<<blocks_for(dm.B), kThreads, 0, st>>>(dm, d.qk, d.bp, mode);
   launch_vertex_rhs<T>(blocks_for(dm.N), kThreads, st, dm, d.qk, d.v, d.cstep, d.bp,
                        std::max(h->prm.air_damping, 0.), d.c.slot_of, d.c.f, b, h->prm.time_step, mode);
@@ -811,10 +816,11 @@ void launch_iteration(pdf_handle* h, T* b, T* y, T* x, const T* Wf, const T* Wb,
 }
 
 // Kernels of this library launched by one PD iteration (CUB's not counted):
-// [bending], vertex rhs, friction, [self friction], forward, backward (small
+// [bending, on large scenes], vertex rhs, friction, [self friction], forward, backward (small
 // scenes: one product), AC.
 int64_t launches_per_iteration(const pdf_handle* h) {
-  return (h->d.dense ? 4 : 5) + (h->dm.B > 0 ? 1 : 0) + (h->prm.self_collision ? 1 : 0);
+  return (h->d.dense ? 4 : 5) + (h->dm.B > 0 && h->dm.N > kFusedLocal ? 1 : 0) +
+         (h->prm.self_collision ? 1 : 0);
 }
 
 // Per step outside the iterations: predictor, obstacle flags + clamp + materialise,

@@ -173,6 +173,14 @@ template <typename T>
 void launch_vertex_rhs(dim3 grid, dim3 block, cudaStream_t st, DModel m, const double* qk, const double* v,
                        const double* cstep, const double* bp, double air_damping, const int* slot_of, double* fslot,
                        T* b, double dt, int residual_mode);
+// Bending projections and right-hand side in one launch, for scenes of up to
+// kFusedLocal vertices: above it the rows computed again for each neighbour cost
+// more than the launch saved (local step alone, two launches in brackets: 900
+// vertices 11.5 us (17.1), 9.4k 13.1 us (16.9), 22.5k 17.6 us (16.7), 40k 23 us (18)).
+constexpr int kFusedLocal = 16384;
+template <typename T>
+void launch_local_fused(cudaStream_t st, DModel m, const double* qk, const double* v, const double* cstep,
+                        double air_damping, const int* slot_of, double* fslot, T* b, double dt, int residual_mode);
 // The contact kernels take the iteration index from *iter: the parity selects
 // the current / next self-contact force buffers, and iteration 0 uses the
 // learned prediction when pred is given.

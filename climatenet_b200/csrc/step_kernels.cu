@@ -45,15 +45,13 @@ __global__ void k_step_init(DModel m, const double* __restrict__ q, double* __re
   }
 }
 
-// Bending projections (BendingConstraint::addConstraintProjection,
+// Bending projection of row b (BendingConstraint::addConstraintProjection,
 // BendingConstraint.cpp:106-138): p_b = sqrt(b) * (rest/|L x|) L x, or 0 when
 // |L x| <= 1e-25, with L x the mean-value Laplacian at the current iterate.
-// Residual mode (FP32 solves) writes p_b - A_b x instead (A_b x = sqrt(b) L x),
+// Residual mode (FP32 solves): p_b - A_b x instead (A_b x = sqrt(b) L x),
 // the row's part of the bending force A_b^T (p_b - A_b x).
-__global__ void k_bend_proj(DModel m, const double* __restrict__ qk, double* __restrict__ bp, int residual_mode) {
-  trace_stamp(m.trace, DTrace::kLocal);
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= m.B) return;
+__device__ __forceinline__ double3 bend_projection(const DModel& m, const double* __restrict__ qk, int b,
+                                                   int residual_mode) {
   double3 lb = make_double3(0., 0., 0.);
   for (int k = m.bend_ptr[b]; k < m.bend_ptr[b + 1]; ++k) lb = lb + m.bend_coef[k] * ld3(qk, m.bend_idx[k]);
   const double n = sqrt(dot3(lb, lb));
@@ -64,7 +62,14 @@ __global__ void k_bend_proj(DModel m, const double* __restrict__ qk, double* __r
     p = w * make_double3(lb.x * s, lb.y * s, lb.z * s);
   }
   if (residual_mode) p = p - w * lb;
-  st3(bp, b, p);
+  return p;
+}
+
+__global__ void k_bend_proj(DModel m, const double* __restrict__ qk, double* __restrict__ bp, int residual_mode) {
+  trace_stamp(m.trace, DTrace::kLocal);
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= m.B) return;
+  st3(bp, b, bend_projection(m, qk, b, residual_mode));
 }
 
 // Vertex-centric local step + right-hand side (SimulationBase::computeProjections
@@ -153,6 +158,101 @@ template void launch_vertex_rhs<double>(dim3, dim3, cudaStream_t, DModel, const 
                                         const double*, double, const int*, double*, double*, double, int);
 template void launch_vertex_rhs<float>(dim3, dim3, cudaStream_t, DModel, const double*, const double*, const double*,
                                        const double*, double, const int*, double*, float*, double, int);
+
+// Local step of small scenes in one launch: 8 lanes a vertex.  Task 0 of a
+// vertex is its own bending row, task k its k-th neighbour: the spring, and the
+// neighbour's bending row, computed here again for each of its neighbours instead
+// of read from k_bend_proj's array.  Three lanes then add the tasks up, one
+// component each, in the order k_vertex_rhs adds them.
+//
+// Bound by latency (the gathers of a row, square roots and divisions) as long as
+// the chip is not full of vertices: the two launches then cost more than the
+// rows computed sevenfold.
+struct LocalTask {
+  double e[3], d[3], p[3];  // spring direction, edge, bending projection
+  double kappa, coef;       // spring and bending coefficients
+  int bend, pad;            // the row exists
+};
+constexpr int kLocalLanes = 8, kLocalThreads = 128, kLocalVerts = kLocalThreads / kLocalLanes;
+template <typename T>
+__global__ void __launch_bounds__(kLocalThreads)
+    k_local(DModel m, const double* __restrict__ qk, const double* __restrict__ v, const double* __restrict__ cstep,
+            double air_damping, const int* __restrict__ slot_of, double* __restrict__ fslot, T* __restrict__ b,
+            double dt, int residual_mode) {
+  trace_stamp(m.trace, DTrace::kLocal);
+  __shared__ LocalTask tasks[kLocalVerts][kLocalLanes];
+  const int lane = threadIdx.x % kLocalLanes, g = threadIdx.x / kLocalLanes;
+  const unsigned int mask = 0xffu << (threadIdx.x & 31 & ~7);
+  const int i = blockIdx.x * kLocalVerts + g;
+  if (i >= m.N) return;
+  const double3 qi = ld3(qk, i);
+  const int r0 = m.ring_ptr[i], n = m.ring_ptr[i + 1] - r0 + 1;
+  const int c = min(lane, 2);  // lanes 0 - 2: their component
+  const double ks = residual_mode ? m.spring_k[i] : 0.;
+  double acc = 0.;
+  for (int t0 = 0; t0 < n; t0 += kLocalLanes) {
+    const int t = t0 + lane;
+    if (t < n) {
+      LocalTask& task = tasks[g][lane];
+      int row;
+      if (t == 0) {
+        row = m.bend_of[i];
+        task.coef = m.self_bend[i];
+      } else {
+        const int s = r0 + t - 1, j = m.ring_idx[s];
+        row = m.bend_of[j];
+        task.coef = m.ring_bend[s];
+        task.kappa = m.ring_kappa[s];
+        const double3 d = qi - ld3(qk, j);
+        st3(task.d, 0, d);
+        st3(task.e, 0, normalized3(d));
+      }
+      task.bend = row >= 0;
+      if (row >= 0) st3(task.p, 0, bend_projection(m, qk, row, residual_mode));
+    }
+    __syncwarp(mask);
+    for (int k = 0; k < min(kLocalLanes, n - t0); ++k) {
+      const LocalTask& task = tasks[g][k];
+      if (t0 + k > 0) {
+        acc = acc + task.kappa * task.e[c];
+        if (residual_mode) acc = acc - ks * task.d[c];
+      }
+      if (task.bend) acc = acc + task.coef * task.p[c];
+    }
+    __syncwarp(mask);
+  }
+  if (lane > 2) return;
+  const int64_t d = 3 * (int64_t)i + c;
+  const double vi = v[d];
+  const int slot = slot_of[i];
+  // air damping is switched off at every contact vertex (SimulationBase.cpp:347-396)
+  const double di = slot >= 0 ? 0. : air_damping;
+  double out;
+  if (residual_mode) {
+    if (m.pin_term) acc = acc + (m.pin_term[d] - m.pin_w[i] * (c == 0 ? qi.x : c == 1 ? qi.y : qi.z));
+    const double mi = m.mass[i];
+    out = mi * (m.tn[d] - vi) + dt * (acc - di * vi);
+    if (slot >= 0) fslot[3 * (int64_t)slot + c] = out + mi * vi;
+  } else {
+    out = cstep[d] + dt * (acc - di * vi);
+    if (slot >= 0) {
+      double a = 0;
+      for (int k = m.ata_ptr[i]; k < m.ata_ptr[i + 1]; ++k) a += m.ata_val[k] * v[3 * (int64_t)m.ata_col[k] + c];
+      fslot[3 * (int64_t)slot + c] = out - dt * dt * a;
+    }
+  }
+  b[m.iperm[i] + (int64_t)c * m.N] = (T)out;
+}
+template <typename T>
+void launch_local_fused(cudaStream_t st, DModel m, const double* qk, const double* v, const double* cstep,
+                        double air_damping, const int* slot_of, double* fslot, T* b, double dt, int residual_mode) {
+  k_local<T><<<(m.N + kLocalVerts - 1) / kLocalVerts, kLocalThreads, 0, st>>>(m, qk, v, cstep, air_damping, slot_of,
+                                                                              fslot, b, dt, residual_mode);
+}
+template void launch_local_fused<double>(cudaStream_t, DModel, const double*, const double*, const double*, double,
+                                         const int*, double*, double*, double, int);
+template void launch_local_fused<float>(cudaStream_t, DModel, const double*, const double*, const double*, double,
+                                        const int*, double*, float*, double, int);
 
 // Adds g into entry p of the three planes (stride n) of a solve vector.
 __device__ __forceinline__ void atomic_add3(double* b, int64_t p, int n, double3 g) {

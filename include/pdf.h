@@ -434,7 +434,7 @@ int pdf_detect_self_collisions(const double* positions, int32_t n_vertices,
  * the reference.  For callers that must not allocate device memory when they
  * detect (code inside another framework's memory pool, real-time loops with a
  * fixed memory budget, hosts whose allocator is not the CUDA runtime's): the
- * whole workspace is one fixed, file-scope device array (about 23 MB, held by
+ * whole workspace is one fixed, file-scope device array (about 22 MB, held by
  * every GPU that loads this library until the process exits); the call makes
  * no cudaMalloc / cudaFree and no allocating library call.
  *   positions (3*n_vertices doubles), triangles (3*n_triangles) and pairs
