@@ -585,8 +585,8 @@ void launch_solve_with(pdf_handle* h, const SweepSync& sy, T* b, T* y, T* x, con
 }
 
 // Small scenes (kDenseBytes): the explicit inverse, its columns three at a time
-// by the FP64 sweeps (whatever the precision of the solve), one captured solve
-// replayed.  false where the scene is too large.
+// by the FP64 sweeps (whatever the precision of the solve), a captured set of
+// solves replayed.  false where the scene is too large.
 bool build_dense(pdf_handle* h) {
   DeviceBuffers& d = h->d;
   const Factor& f = h->fac;
@@ -614,60 +614,77 @@ bool build_dense(pdf_handle* h) {
   else
     d.dense64 = dalloc<double>(total);
   CK(cudaMemsetAsync(h->fp32 ? (void*)d.dense32 : (void*)d.dense64, 0, total * s, st));  // the rows' padding
-  // FP64 sweeps on scratch vectors (the handle's own where it solves in FP64)
+  // FP64 sweeps, kBranches of them side by side (each is a chain of short
+  // launches): vectors, queues, solve counter and column of their own
+  constexpr int kBranches = 4;
   const bool fp32 = h->fp32;
   std::vector<void*> tmp;
-  auto scratch = [&](size_t n) {
-    double* p = dalloc<double>(n);
-    tmp.push_back(p);
-    return p;
-  };
-  double *Wf = d.Wf64, *Wb = d.Wb64, *b = d.b64, *y = d.y64, *x = d.x64;
-  double *v = nullptr, *qk = nullptr;
+  cudaStream_t side[kBranches] = {};
+  cudaEvent_t ev[kBranches] = {};
   cudaGraphExec_t exec = nullptr;
-  int* column = nullptr;
   auto release = [&] {
     if (exec) cudaGraphExecDestroy(exec);
-    if (column) cudaFree(column);
     for (void* p : tmp) cudaFree(p);
+    for (cudaStream_t s2 : side)
+      if (s2) cudaStreamDestroy(s2);
+    for (cudaEvent_t e2 : ev)
+      if (e2) cudaEventDestroy(e2);
     h->fp32 = fp32;
   };
   try {
     h->fp32 = false;
     // leaves and their parents as blocks, 32-column items, 2 CTAs of 8 warps
     build_schedule(h, 32, 1, 1, 1);
+    double *Wf = d.Wf64, *Wb = d.Wb64;
     if (fp32) {
       tmp.push_back(Wf = upload(f.Wf));
       tmp.push_back(Wb = upload(f.Wb));
-      b = scratch(3 * (size_t)N);
-      y = scratch(3 * (size_t)N);
-      x = scratch(3 * (size_t)N);
     }
-    v = scratch(3 * (size_t)N);
-    qk = scratch(3 * (size_t)N);
-    column = dalloc<int>(1);
-    CK(cudaMemsetAsync(column, 0, sizeof(int), st));
-    SweepSync sy = d.sync;
-    sy.trace.stamps = nullptr;
-    launch_solve_prep<double>(st, N, x, y, sy);
+    double* vec[kBranches];  // b, y, x, v, q^k
+    int* column[kBranches];
+    SweepSync sy[kBranches];
+    const size_t n3 = 3 * (size_t)N;
+    for (int k = 0; k < kBranches; ++k) {
+      tmp.push_back(vec[k] = dalloc<double>(5 * n3));
+      tmp.push_back(column[k] = dalloc<int>(1));
+      const int first = 3 * k;
+      CK(cudaMemcpyAsync(column[k], &first, sizeof(int), cudaMemcpyHostToDevice, st));
+      sy[k] = d.sync;
+      sy[k].trace.stamps = nullptr;
+      tmp.push_back(sy[k].queue = dalloc<int>(4));
+      tmp.push_back(sy[k].epoch = dalloc<unsigned long long>(1));
+      CK(cudaMemsetAsync(sy[k].epoch, 0, sizeof(unsigned long long), st));
+      launch_solve_prep<double>(st, N, vec[k] + 2 * n3, vec[k] + n3, sy[k]);
+      CK(cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming));
+      if (k > 0) CK(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking));
+    }
     cudaGraph_t g;
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    launch_dense_unit(st, d.dense_rows, b, N, column);
-    launch_solve_sweeps<double>(st, d.plan, Wf, Wb, b, y, x, N, sy, WriteBack{v, qk, d.q, 0., 0});
-    if (fp32)
-      launch_dense_rows<float>(st, d.dense_rows, v, N, d.perm, d.dense32, column);
-    else
-      launch_dense_rows<double>(st, d.dense_rows, v, N, d.perm, d.dense64, column);
+    cudaEventRecord(ev[0], st);
+    for (int k = 0; k < kBranches; ++k) {
+      cudaStream_t s2 = k > 0 ? side[k] : st;
+      if (k > 0) cudaStreamWaitEvent(s2, ev[0], 0);
+      double *b = vec[k], *y = b + n3, *x = y + n3, *v = x + n3, *qk = v + n3;
+      launch_dense_unit(s2, d.dense_rows, b, N, column[k]);
+      launch_solve_sweeps<double>(s2, d.plan, Wf, Wb, b, y, x, N, sy[k], WriteBack{v, qk, d.q, 0., 0});
+      if (fp32)
+        launch_dense_rows<float>(s2, d.dense_rows, v, N, d.perm, d.dense32, column[k], 3 * kBranches);
+      else
+        launch_dense_rows<double>(s2, d.dense_rows, v, N, d.perm, d.dense64, column[k], 3 * kBranches);
+      if (k > 0) cudaEventRecord(ev[k], s2);
+    }
+    for (int k = 1; k < kBranches; ++k) cudaStreamWaitEvent(st, ev[k], 0);
     CK(cudaStreamEndCapture(st, &g));
     const cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
     CK(e);
-    for (int k = 0; k < widest; k += 3) CK(cudaGraphLaunch(exec, st));
+    for (int k = 0; k < widest; k += 3 * kBranches) CK(cudaGraphLaunch(exec, st));
     CK(cudaStreamSynchronize(st));
     int derr = 0;
     CK(cudaMemcpy(&derr, d.sync.err, sizeof(int), cudaMemcpyDeviceToHost));
     if (derr) throw CudaFail("a supernodal sweep gave up waiting while the inverse was built");
   } catch (...) {
+    cudaStreamSynchronize(st);
     release();
     throw;
   }

@@ -144,18 +144,19 @@ __global__ void k_dense_rows(const DenseRow* __restrict__ rows, const double* __
       if (k + c < rows[i].n) A[rows[c0 + k + c].off + i - c0] = (T)v[3 * (int64_t)perm[i] + c];
   }
 }
-__global__ void k_dense_next(int* column) { *column += 3; }
+__global__ void k_dense_next(int* column, int step) { *column += step; }
 
 void launch_dense_unit(cudaStream_t st, const DenseRow* rows, double* b, int n, const int* column) {
   k_dense_unit<<<std::min(148, (n + 255) / 256), 256, 0, st>>>(rows, b, n, column);
 }
 template <typename T>
 void launch_dense_rows(cudaStream_t st, const DenseRow* rows, const double* v, int n, const int* perm, T* A,
-                       int* column) {
+                       int* column, int step) {
   k_dense_rows<T><<<std::min(148, (n + 255) / 256), 256, 0, st>>>(rows, v, n, perm, A, column);
-  k_dense_next<<<1, 1, 0, st>>>(column);
+  k_dense_next<<<1, 1, 0, st>>>(column, step);
 }
-template void launch_dense_rows<double>(cudaStream_t, const DenseRow*, const double*, int, const int*, double*, int*);
-template void launch_dense_rows<float>(cudaStream_t, const DenseRow*, const double*, int, const int*, float*, int*);
+template void launch_dense_rows<double>(cudaStream_t, const DenseRow*, const double*, int, const int*, double*, int*,
+                                        int);
+template void launch_dense_rows<float>(cudaStream_t, const DenseRow*, const double*, int, const int*, float*, int*, int);
 
 }  // namespace pdfb

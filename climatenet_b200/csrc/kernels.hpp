@@ -225,7 +225,7 @@ bool launch_dense_solve(cudaStream_t st, const DenseRow* rows, const T* A, const
 void launch_dense_unit(cudaStream_t st, const DenseRow* rows, double* b, int n, const int* column);
 template <typename T>
 void launch_dense_rows(cudaStream_t st, const DenseRow* rows, const double* v, int n, const int* perm, T* A,
-                       int* column);
+                       int* column, int step);  // then *column += step
 
 // detection (detect_kernels.cu, compiled without FMA contraction)
 __global__ void k_obstacle_flags(int N, const double* q, DObstacles obs, unsigned char* flags);
