@@ -701,9 +701,10 @@ bool build_dense(pdf_handle* h) {
 }
 
 // Schedule autotuner: times the global solve of this scene's factor with
-// each candidate cut level and both upper modes (work-item width 64, block
+// each candidate cut level (work-item width 32, level launches, block
 // kernels at 2 CTAs of 8 or 4 CTAs of 4 consumer warps per SM where they
-// fit), then with each launch shape of the block kernels at the best cut
+// fit; dependency-driven upper items, the slower mode, only where the levels do
+// not fit the launch table), then with each launch shape of the block kernels at the best cut
 // level and mode, then with each work-item width, and keeps the fastest.  The right-hand side is
 // zero (the sweeps read the same data and wait on the same dependencies
 // whatever the values); v and q^k, which the solve writes, are restored.
@@ -719,8 +720,8 @@ void autotune_schedule(pdf_handle* h) {
   auto time_plan = [&](int chunk, int cut, int mode, int shape, bool exact_shape) {
     build_schedule(h, chunk, cut, mode, shape);
     if (h->d.plan.upper_mode != mode || (exact_shape && h->d.plan.block_shape != shape)) return 0.;
-    double total = 0.;
-    for (int r = 0; r < 4; ++r) {
+    double fastest = 1e300;
+    for (int r = 0; r < 5; ++r) {
       if (h->fp32) {
         CK(cudaMemsetAsync(d.b32, 0, 3 * (size_t)N * sizeof(float), st));
         launch_solve_prep<float>(st, N, d.x32, d.y32, d.sync);
@@ -737,52 +738,45 @@ void autotune_schedule(pdf_handle* h) {
       CK(cudaEventSynchronize(h->ev[6]));
       float ms = 0.f;
       CK(cudaEventElapsedTime(&ms, h->ev[5], h->ev[6]));
-      if (r > 0) total += ms;  // first run warms up
+      if (r > 0) fastest = std::min(fastest, (double)ms);  // first run warms up
     }
     int derr = 0;
     CK(cudaMemcpy(&derr, d.sync.err, sizeof(int), cudaMemcpyDeviceToHost));
     if (derr) throw CudaFail("a supernodal sweep gave up waiting for a dependency while tuning");
-    return total / 3.;
+    return fastest;
   };
   double best = 1e300;
   int best_cut = kCutLevel, best_chunk = kChunk, best_mode = 0, best_shape = kBlockShape;
   double cut_ms[2][kCutCandidates] = {};
-  int cut_shape[2][kCutCandidates] = {};
+  auto consider = [&](int cut, int mode, int sh, bool exact_shape) {
+    const double ms = time_plan(kChunk, cut, mode, sh, exact_shape);
+    if (ms <= 0.) return;
+    if (cut_ms[mode][cut] == 0. || ms < cut_ms[mode][cut]) cut_ms[mode][cut] = ms;
+    if (ms < best) {
+      best = ms;
+      best_cut = cut;
+      best_mode = mode;
+      best_shape = h->d.plan.block_shape;
+    }
+  };
   for (int cut = 0; cut < kCutCandidates; ++cut)
-    for (int mode = 0; mode < 2; ++mode)
-      for (int sh : kStageOneShapes) {
-        const double ms = time_plan(kChunk, cut, mode, sh, true);
-        if (ms > 0. && (cut_ms[mode][cut] == 0. || ms < cut_ms[mode][cut])) {
-          cut_ms[mode][cut] = ms;
-          cut_shape[mode][cut] = sh;
-        }
-        if (ms > 0. && ms < best) {
-          best = ms;
-          best_cut = cut;
-          best_mode = mode;
-        }
-      }
-  if (best == 1e300) {  // neither first-stage shape fits any cut: one CTA of 8 warps
+    for (int sh : kStageOneShapes) consider(cut, 1, sh, true);
+  // dependency-driven items where the levels exceed the launch table, and one
+  // CTA of 8 warps where neither first-stage shape fits any cut
+  if (best == 1e300)
     for (int cut = 0; cut < kCutCandidates; ++cut)
-      for (int mode = 0; mode < 2; ++mode) {
-        const double ms = time_plan(kChunk, cut, mode, 0, false);
-        cut_ms[mode][cut] = ms;
-        cut_shape[mode][cut] = h->d.plan.block_shape;
-        if (ms > 0. && ms < best) {
-          best = ms;
-          best_cut = cut;
-          best_mode = mode;
-        }
-      }
-  }
+      for (int sh : kStageOneShapes) consider(cut, 0, sh, true);
+  if (best == 1e300)
+    for (int cut = 0; cut < kCutCandidates; ++cut)
+      for (int mode = 0; mode < 2; ++mode) consider(cut, mode, 0, false);
   for (int cut = 0; cut < kCutCandidates; ++cut) {
     h->stats.sweep_cut_ms[cut] = cut_ms[0][cut];
     h->stats.sweep_cut_level_ms[cut] = cut_ms[1][cut];
   }
   // the block kernels' launch shapes at the best cut level and mode
-  best_shape = cut_shape[best_mode][best_cut];
+  const int first_shape = best_shape;
   for (int sh = 0; sh < kBlockShapes; ++sh) {
-    const double ms = sh == best_shape ? best : time_plan(kChunk, best_cut, best_mode, sh, true);
+    const double ms = sh == first_shape ? best : time_plan(kChunk, best_cut, best_mode, sh, true);
     h->stats.sweep_shape_ms[sh] = ms;
     if (ms > 0. && ms < best) {
       best = ms;

@@ -187,7 +187,8 @@ typedef struct pdf_stats {
    * the number of blocks, and the factor elements in blocks / above them */
   int32_t sweep_cut_level, sweep_blocks;
   int64_t sweep_block_elems, sweep_upper_elems;
-  double sweep_cut_ms[8];           /* solve time measured for cut levels 0-7   */
+  double sweep_cut_ms[8];           /* solve time in mode 0 for cut levels 0-7
+                                       (0 where not timed: mode 1 could run)    */
   /* the supernodes above the blocks: 0 = dependency-driven work items in one
    * launch per sweep, 1 = one launch per elimination-tree level; the number
    * of such levels, and the solve time in mode 1 for cut levels 0-7 (0 where
