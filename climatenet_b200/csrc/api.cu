@@ -586,7 +586,7 @@ void launch_solve_with(pdf_handle* h, const SweepSync& sy, T* b, T* y, T* x, con
 
 // Small scenes (kDenseBytes): the explicit inverse, its columns three at a time
 // by the FP64 sweeps (whatever the precision of the solve), a captured set of
-// solves replayed.  false where the scene is too large.
+// solves replayed.  false where the scene is too large, or memory too short.
 bool build_dense(pdf_handle* h) {
   DeviceBuffers& d = h->d;
   const Factor& f = h->fac;
@@ -608,11 +608,16 @@ bool build_dense(pdf_handle* h) {
   if (3 * (size_t)np * s > (size_t)kDenseSmem) return false;
   d.dense_np = np;
   cudaStream_t st = h->stream;
-  d.dense_rows = upload(rows);
+  void* mem = nullptr;
+  if (cudaMalloc(&mem, total * s) != cudaSuccess) {  // no room for it: the sweeps
+    cudaGetLastError();
+    return false;
+  }
   if (h->fp32)
-    d.dense32 = dalloc<float>(total);
+    d.dense32 = (float*)mem;
   else
-    d.dense64 = dalloc<double>(total);
+    d.dense64 = (double*)mem;
+  d.dense_rows = upload(rows);
   CK(cudaMemsetAsync(h->fp32 ? (void*)d.dense32 : (void*)d.dense64, 0, total * s, st));  // the rows' padding
   // FP64 sweeps, kBranches of them side by side (each is a chain of short
   // launches): vectors, queues, solve counter and column of their own

@@ -180,7 +180,10 @@ typedef struct pdf_stats {
   int32_t n_constraint_rows;        /* rows(A)                                  */
   int64_t kernel_launches;          /* this library's kernels launched so far   */
   int64_t factor_nnz_true;          /* structural nnz(L) without padding        */
-  int32_t sweep_chunk;              /* work-item width chosen by the autotuner  */
+  int32_t sweep_chunk;              /* work-item width chosen by the autotuner
+                                       (scenes solved by one product with the
+                                       inverse: sweep_* are the schedule of the
+                                       sweeps it stands in for, times 0)        */
   double sweep_chunk_ms[3];         /* solve time measured for 32, 64, 128      */
   /* subtree blocks of the solve schedule chosen by the autotuner: the
    * elimination-tree level up to which subtrees are solved by one CTA each,
