@@ -171,6 +171,19 @@ void build_schedule(pdf_handle* h, int chunk, int cut_level, int upper_mode = 0,
 void autotune_schedule(pdf_handle* h);
 bool build_dense(pdf_handle* h);
 
+// Whether the inverses of components of these sizes are kept (kDenseBytes, kDenseSmem).
+bool dense_fits(const std::vector<int>& sizes, size_t elem) {
+  const uint64_t pad = 16 / elem;
+  uint64_t total = 0, np = 0;
+  for (int n : sizes) {
+    const uint64_t ld = (n + pad - 1) / pad * pad;
+    np += ld;
+    total += n * ld;
+    if (total > kDenseBytes / elem) return false;
+  }
+  return 3 * np * elem <= (uint64_t)kDenseSmem;
+}
+
 // Warm-start feature / prediction buffers and the impulse memory.
 void ensure_mlp_buffers(pdf_handle* h) {
   if (h->mlp_X) return;
@@ -243,7 +256,8 @@ void create_impl(pdf_handle* h, const pdf_scene_desc* sc, const pdf_params* p) {
   h->lhs_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tl).count();
   const Model& m = h->model;
   std::string ferr;
-  if (!factorize(m, p->time_step, 40, h->fac, ferr)) throw std::range_error(ferr);
+  auto inverse_fits = [](const std::vector<int>& sizes) { return dense_fits(sizes, sizeof(float)); };
+  if (!factorize(m, p->time_step, 40, h->fac, ferr, h->fp32 ? +inverse_fits : nullptr)) throw std::range_error(ferr);
   const Factor& f = h->fac;
   const int N = m.N;
   CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
@@ -596,16 +610,16 @@ bool build_dense(pdf_handle* h) {
   std::vector<DenseRow> rows(N);
   int64_t total = 0;
   int widest = 0, np = 0;
+  std::vector<int> sizes;
+  for (size_t c = 0; c + 1 < f.comp_ptr.size(); ++c) sizes.push_back(f.comp_ptr[c + 1] - f.comp_ptr[c]);
+  if (!dense_fits(sizes, s)) return false;
   for (size_t c = 0; c + 1 < f.comp_ptr.size(); ++c) {
     const int c0 = f.comp_ptr[c], n = f.comp_ptr[c + 1] - c0, ld = (n + pad - 1) / pad * pad;
-    if ((uint64_t)n * ld > kDenseBytes / s) return false;
     for (int r = 0; r < n; ++r) rows[c0 + r] = DenseRow{total + (int64_t)r * ld, c0, n, np - c0};
     np += ld;
     total += (int64_t)n * ld;
     widest = std::max(widest, n);
-    if ((uint64_t)total > kDenseBytes / s) return false;
   }
-  if (3 * (size_t)np * s > (size_t)kDenseSmem) return false;
   d.dense_np = np;
   cudaStream_t st = h->stream;
   void* mem = nullptr;

@@ -3,6 +3,7 @@
 #include "factor.hpp"
 
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <cstdint>
 #include <stdexcept>
@@ -130,6 +131,53 @@ std::vector<std::vector<int>> components(const Model& m) {
   return out;
 }
 
+// The components whose bounding boxes overlap (layers) united, vertices ascending.
+std::vector<std::vector<int>> united(const Model& m, const std::vector<std::vector<int>>& comps) {
+  const int n = (int)comps.size();
+  std::vector<std::array<double, 6>> box(n);
+  for (int c = 0; c < n; ++c) {
+    box[c] = {1e300, 1e300, 1e300, -1e300, -1e300, -1e300};
+    for (int v : comps[c])
+      for (int k = 0; k < 3; ++k) {
+        box[c][k] = std::min(box[c][k], m.rest[3 * (size_t)v + k]);
+        box[c][3 + k] = std::max(box[c][3 + k], m.rest[3 * (size_t)v + k]);
+      }
+  }
+  std::vector<int> set(n), by_x(n);
+  std::iota(set.begin(), set.end(), 0);
+  std::iota(by_x.begin(), by_x.end(), 0);
+  auto root = [&](int c) {
+    while (set[c] != c) c = set[c] = set[set[c]];
+    return c;
+  };
+  std::sort(by_x.begin(), by_x.end(), [&](int a, int b) { return box[a][0] < box[b][0]; });
+  for (int i = 0; i < n; ++i)
+    for (int j = i + 1; j < n && box[by_x[j]][0] <= box[by_x[i]][3]; ++j) {
+      const auto &a = box[by_x[i]], &b = box[by_x[j]];
+      // in the plane of the two widest extents layers cover each other; along the
+      // third they may lie apart
+      int over = 0;
+      double gap = 0., side = 0.;
+      for (int k = 0; k < 3; ++k) {
+        if (a[k] <= b[3 + k] && b[k] <= a[3 + k]) ++over;
+        gap = std::max(gap, std::max(a[k] - b[3 + k], b[k] - a[3 + k]));
+        side = std::max(side, std::min(a[3 + k] - a[k], b[3 + k] - b[k]));
+      }
+      if (over == 3 || (over == 2 && gap < 0.05 * side)) {
+        const int ra = root(by_x[i]), rb = root(by_x[j]);
+        set[std::max(ra, rb)] = std::min(ra, rb);
+      }
+    }
+  std::vector<std::vector<int>> out(n);
+  for (int c = 0; c < n; ++c) {
+    auto& ids = out[root(c)];
+    ids.insert(ids.end(), comps[c].begin(), comps[c].end());
+  }
+  out.erase(std::remove_if(out.begin(), out.end(), [](const auto& ids) { return ids.empty(); }), out.end());
+  for (auto& ids : out) std::sort(ids.begin(), ids.end());
+  return out;
+}
+
 // Top dissection levels merged into the root supernode (PDF_ND_MERGE
 // overrides it for tuning experiments).  A merged level saves a launch per sweep
 // (some 3 us each) and fills the root: by 40 N entries from three levels to four, by
@@ -178,7 +226,8 @@ bool blocked_cholesky(double* F, int ns, int ld) {
 
 }  // namespace
 
-bool factorize(const Model& m, double dt, int leaf_size, Factor& f, std::string& err) {
+bool factorize(const Model& m, double dt, int leaf_size, Factor& f, std::string& err,
+               bool (*apart)(const std::vector<int>& sizes)) {
   auto t_start = std::chrono::steady_clock::now();
   const int N = m.N;
   f.N = N;
@@ -188,8 +237,16 @@ bool factorize(const Model& m, double dt, int leaf_size, Factor& f, std::string&
     // each connected component of the matrix graph (a layer, a cloth of a
     // batch) on its own: dissected together, components that overlap in space
     // share supernodes, whose dense blocks hold a zero for every pair of rows of
-    // different components (three 128 x 128 layers: 16.5 M stored entries against 6.1 M)
-    for (std::vector<int>& ids : components(m)) {
+    // different components (three 128 x 128 layers: 16.5 M stored entries against 6.1 M).
+    // FP32 sweeps (`apart`) keep layers together: apart, their result was further
+    // from the FP64 solve's by a fifth (two 256 x 256 layers, one step of 20
+    // iterations, six inputs: 2.2e-6 to 2.4e-6
+    // relative against 2.0e-6), for all that a solve took 0.105 ms instead of 0.136
+    std::vector<std::vector<int>> comps = components(m);
+    std::vector<int> sizes;
+    for (const std::vector<int>& ids : comps) sizes.push_back((int)ids.size());
+    if (apart && comps.size() > 1 && !apart(sizes)) comps = united(m, comps);
+    for (std::vector<int>& ids : comps) {
       f.comp_ptr.push_back((int)nd.order.size());
       nd.run(ids);
       nd.top();

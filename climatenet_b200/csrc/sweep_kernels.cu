@@ -21,8 +21,8 @@
 //     on the data).  The ext rows' updates are added to b with one atomic
 //     each per block.
 //  2. the supernodes above the blocks, forward, split into 32-row tiles x
-//     column chunks: either k_upper_level_forward, one launch per
-//     elimination-tree level (items spread over all warps, the launch
+//     column chunks: either k_upper_level, one launch per elimination-tree
+//     level (its tiles brought to shared memory by bulk copies, the launch
 //     boundary ordering the levels), or k_upper_forward, one launch whose
 //     warps take items from a queue in elimination-tree order and wait
 //     (bounded spin) until every work item of the supernode's upper children
