@@ -164,8 +164,11 @@ __device__ __forceinline__ void stage_items(BlockItem* dst, const BlockItem* src
   }
 }
 
-// Block tickets: thread 0 draws the first one before the loop and the next
-// one when a block enters its last level (its round trip overlaps that
+// Block tickets: the forward sweep's thread 0 draws the first one before the
+// loop, the backward sweep's first one is the CTA's index (that launch is a
+// programmatic dependent: before its wait it must not touch the queue, which
+// the forward launch rewinds, and nothing would order the two); the next one is
+// drawn when a block enters its last level (its round trip overlaps that
 // level, and blocks are still claimed in about the order CTAs free up); the
 // ticket is published in shared memory between two barriers at the block's
 // end, after every thread has read the current one.
@@ -595,8 +598,10 @@ __global__ void __launch_bounds__(kBlockMaxThreads, 1) k_block_backward(DPlan P,
   int q_base = 0, q_issued = 0;
   bool failed = false;
   int next_ticket = 0;  // thread 0
+  // the first blocks go by CTA: the queue, which the forward sweep's launch
+  // rewinds, is only read behind griddep_wait()
   if (threadIdx.x == 0) {
-    s_ticket = atomicAdd(sy.queue + 3, 1);
+    s_ticket = blockIdx.x;
     s_failed = 0;
   }
   __syncthreads();
@@ -661,7 +666,7 @@ __global__ void __launch_bounds__(kBlockMaxThreads, 1) k_block_backward(DPlan P,
       failed = failed || !__shfl_sync(0xffffffffu, ok, 0);
     } else {
       for (int L = 0; L < nlev; ++L) {
-        if (L == nlev - 1 && threadIdx.x == 0) next_ticket = atomicAdd(sy.queue + 3, 1);
+        if (L == nlev - 1 && threadIdx.x == 0) next_ticket = gridDim.x + atomicAdd(sy.queue + 3, 1);
         const int i1 = s_lev[L + 1];
 #pragma unroll 1
         for (int it = s_lev[L] + warp; it < i1; it += ncw) {
