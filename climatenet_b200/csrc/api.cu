@@ -171,19 +171,6 @@ void build_schedule(pdf_handle* h, int chunk, int cut_level, int upper_mode = 0,
 void autotune_schedule(pdf_handle* h);
 bool build_dense(pdf_handle* h);
 
-// Whether the inverses of components of these sizes are kept (kDenseBytes, kDenseSmem).
-bool dense_fits(const std::vector<int>& sizes, size_t elem) {
-  const uint64_t pad = 16 / elem;
-  uint64_t total = 0, np = 0;
-  for (int n : sizes) {
-    const uint64_t ld = (n + pad - 1) / pad * pad;
-    np += ld;
-    total += n * ld;
-    if (total > kDenseBytes / elem) return false;
-  }
-  return 3 * np * elem <= (uint64_t)kDenseSmem;
-}
-
 // Warm-start feature / prediction buffers and the impulse memory.
 void ensure_mlp_buffers(pdf_handle* h) {
   if (h->mlp_X) return;
@@ -256,8 +243,7 @@ void create_impl(pdf_handle* h, const pdf_scene_desc* sc, const pdf_params* p) {
   h->lhs_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tl).count();
   const Model& m = h->model;
   std::string ferr;
-  auto inverse_fits = [](const std::vector<int>& sizes) { return dense_fits(sizes, sizeof(float)); };
-  if (!factorize(m, p->time_step, 40, h->fac, ferr, h->fp32 ? +inverse_fits : nullptr)) throw std::range_error(ferr);
+  if (!factorize(m, p->time_step, 40, h->fac, ferr, h->fp32)) throw std::range_error(ferr);
   const Factor& f = h->fac;
   const int N = m.N;
   CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
@@ -571,23 +557,25 @@ void launch_local(pdf_handle* h, T* b, int mode) {
                        std::max(h->prm.air_damping, 0.), d.c.slot_of, d.c.f, b, h->prm.time_step, mode);
 }
 
-// The inverse in the precision of the solve (b only picks it).
-inline const double* dense_of(const DeviceBuffers& d, const double*) { return d.dense64; }
-inline const float* dense_of(const DeviceBuffers& d, const float*) { return d.dense32; }
+// The product with the inverse (FP64 solves; b picks the overload).
+inline bool solve_dense(pdf_handle* h, const double* b, const WriteBack& wb) {
+  DeviceBuffers& d = h->d;
+  if (!d.dense) return false;
+  if (!launch_dense_solve(h->stream, d.dense_rows, d.inverse, b, h->dm.N, d.dense_np, d.perm, wb, h->dm.trace))
+    throw CudaFail("the dense solve does not fit the device's shared memory");
+  return true;
+}
+inline bool solve_dense(pdf_handle*, const float*, const WriteBack&) { return false; }
 
-// Global solve: for small scenes one product with the inverse; else one persistent forward and one backward sweep (which writes
-// back v and q^k of the blocks' columns), then the write-back of the upper
-// columns (which also clears their x, y for the next solve).
+// Global solve: for small FP64 scenes one product with the inverse; else the forward
+// and the backward sweep, whose last launch writes v and q^k back.  The sweeps
+// carry state from one solve to the next: x of the upper columns is cleared by the
+// forward block kernel, their y by the backward one behind its wait.
 template <typename T>
 void launch_solve(pdf_handle* h, T* b, T* y, T* x, const T* Wf, const T* Wb, int mode) {
   DeviceBuffers& d = h->d;
   const WriteBack wb{d.v, d.qk, d.q, h->prm.time_step, mode};
-  if (d.dense) {
-    const T* A = dense_of(d, b);
-    if (!launch_dense_solve<T>(h->stream, d.dense_rows, A, b, h->dm.N, d.dense_np, d.perm, wb, h->dm.trace))
-      throw CudaFail("the dense solve does not fit the device's shared memory");
-    return;
-  }
+  if (solve_dense(h, b, wb)) return;
   launch_solve_sweeps<T>(h->stream, d.plan, Wf, Wb, b, y, x, h->dm.N, d.sync, wb);
 }
 
@@ -598,45 +586,39 @@ void launch_solve_with(pdf_handle* h, const SweepSync& sy, T* b, T* y, T* x, con
                          WriteBack{d.v, d.qk, d.q, h->prm.time_step, mode});
 }
 
-// Small scenes (kDenseBytes): the explicit inverse, its columns three at a time
-// by the FP64 sweeps (whatever the precision of the solve), a captured set of
-// solves replayed.  false where the scene is too large, or memory too short.
+// Small FP64 scenes (kDenseBytes): the explicit inverse, its columns three at a
+// time by the sweeps, a captured set of solves replayed.  false where the scene is
+// too large, or memory too short.
 bool build_dense(pdf_handle* h) {
   DeviceBuffers& d = h->d;
   const Factor& f = h->fac;
   const int N = h->dm.N;
-  const size_t s = h->fp32 ? sizeof(float) : sizeof(double);
-  const int pad = 16 / (int)s;
+  if (h->fp32) return false;
   std::vector<DenseRow> rows(N);
-  int64_t total = 0;
-  int widest = 0, np = 0;
-  std::vector<int> sizes;
-  for (size_t c = 0; c + 1 < f.comp_ptr.size(); ++c) sizes.push_back(f.comp_ptr[c + 1] - f.comp_ptr[c]);
-  if (!dense_fits(sizes, s)) return false;
+  int64_t total = 0, np = 0;
+  int widest = 0;
   for (size_t c = 0; c + 1 < f.comp_ptr.size(); ++c) {
-    const int c0 = f.comp_ptr[c], n = f.comp_ptr[c + 1] - c0, ld = (n + pad - 1) / pad * pad;
-    for (int r = 0; r < n; ++r) rows[c0 + r] = DenseRow{total + (int64_t)r * ld, c0, n, np - c0};
+    const int c0 = f.comp_ptr[c], n = f.comp_ptr[c + 1] - c0, ld = (n + 1) / 2 * 2;
+    if ((total + (int64_t)n * ld) * sizeof(double) > kDenseBytes || 3 * (np + ld) * sizeof(double) > kDenseSmem)
+      return false;
+    for (int r = 0; r < n; ++r) rows[c0 + r] = DenseRow{total + (int64_t)r * ld, c0, n, (int)np - c0};
     np += ld;
     total += (int64_t)n * ld;
     widest = std::max(widest, n);
   }
-  d.dense_np = np;
+  d.dense_np = (int)np;
   cudaStream_t st = h->stream;
   void* mem = nullptr;
-  if (cudaMalloc(&mem, total * s) != cudaSuccess) {  // no room for it: the sweeps
+  if (cudaMalloc(&mem, total * sizeof(double)) != cudaSuccess) {  // no room for it: the sweeps
     cudaGetLastError();
     return false;
   }
-  if (h->fp32)
-    d.dense32 = (float*)mem;
-  else
-    d.dense64 = (double*)mem;
+  d.inverse = (double*)mem;
   d.dense_rows = upload(rows);
-  CK(cudaMemsetAsync(h->fp32 ? (void*)d.dense32 : (void*)d.dense64, 0, total * s, st));  // the rows' padding
-  // FP64 sweeps, kBranches of them side by side (each is a chain of short
-  // launches): vectors, queues, solve counter and column of their own
+  CK(cudaMemsetAsync(d.inverse, 0, total * sizeof(double), st));  // the rows' padding
+  // kBranches sweeps side by side (each is a chain of short launches): vectors,
+  // queues, solve counter and column of their own
   constexpr int kBranches = 4;
-  const bool fp32 = h->fp32;
   std::vector<void*> tmp;
   cudaStream_t side[kBranches] = {};
   cudaEvent_t ev[kBranches] = {};
@@ -648,17 +630,10 @@ bool build_dense(pdf_handle* h) {
       if (s2) cudaStreamDestroy(s2);
     for (cudaEvent_t e2 : ev)
       if (e2) cudaEventDestroy(e2);
-    h->fp32 = fp32;
   };
   try {
-    h->fp32 = false;
     // leaves and their parents as blocks, 32-column items, 2 CTAs of 8 warps
     build_schedule(h, 32, 1, 1, 1);
-    double *Wf = d.Wf64, *Wb = d.Wb64;
-    if (fp32) {
-      tmp.push_back(Wf = upload(f.Wf));
-      tmp.push_back(Wb = upload(f.Wb));
-    }
     double* vec[kBranches];  // b, y, x, v, q^k
     int* column[kBranches];
     SweepSync sy[kBranches];
@@ -685,11 +660,8 @@ bool build_dense(pdf_handle* h) {
       if (k > 0) cudaStreamWaitEvent(s2, ev[0], 0);
       double *b = vec[k], *y = b + n3, *x = y + n3, *v = x + n3, *qk = v + n3;
       launch_dense_unit(s2, d.dense_rows, b, N, column[k]);
-      launch_solve_sweeps<double>(s2, d.plan, Wf, Wb, b, y, x, N, sy[k], WriteBack{v, qk, d.q, 0., 0});
-      if (fp32)
-        launch_dense_rows<float>(s2, d.dense_rows, v, N, d.perm, d.dense32, column[k], 3 * kBranches);
-      else
-        launch_dense_rows<double>(s2, d.dense_rows, v, N, d.perm, d.dense64, column[k], 3 * kBranches);
+      launch_solve_sweeps<double>(s2, d.plan, d.Wf64, d.Wb64, b, y, x, N, sy[k], WriteBack{v, qk, d.q, 0., 0});
+      launch_dense_rows(s2, d.dense_rows, v, N, d.perm, d.inverse, column[k], 3 * kBranches);
       if (k > 0) cudaEventRecord(ev[k], s2);
     }
     for (int k = 1; k < kBranches; ++k) cudaStreamWaitEvent(st, ev[k], 0);
@@ -709,11 +681,7 @@ bool build_dense(pdf_handle* h) {
   }
   release();
   // the schedule the sweeps would take, should pdf_set_sweep_schedule ask for them
-  build_schedule(h, 32, 1, 1, 1);
-  if (fp32)
-    launch_solve_prep<float>(st, N, d.x32, d.y32, d.sync);
-  else
-    launch_solve_prep<double>(st, N, d.x64, d.y64, d.sync);
+  launch_solve_prep<double>(st, N, d.x64, d.y64, d.sync);
   CK(cudaStreamSynchronize(st));
   d.dense = true;
   return true;
@@ -1181,7 +1149,7 @@ void free_handle(pdf_handle* h) {
                   d.c.s_ac, d.c.s_slota, d.c.s_slotb, d.c.s_remember, d.c.n_levels, d.c.level_ptr,
                   d.c.level_order, d.c.slot_of, d.c.n_slots, d.c.slot_vertex, d.c.f, d.c.cf[0], d.c.cf[1],
                   d.c.sf[0], d.c.sf[1], d.c.c_gap, d.c.c_active, h->mlp_w, h->mlp_X, h->mlp_Y, h->rprev,
-                  h->rprev_tag, h->log_X, h->log_T, h->log_n, d.iter, d.iter_total, d.blocks_done, d.stamps, d.dense_rows, d.dense64, d.dense32,
+                  h->rprev_tag, h->log_X, h->log_T, h->log_n, d.iter, d.iter_total, d.blocks_done, d.stamps, d.dense_rows, d.inverse,
                   d.c.ac_trace, h->gather_idx, h->gather_out, h->stage, h->bad_dev, d.ob_best};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -1754,10 +1722,7 @@ int pdf_time_solve_parts(pdf_handle* h, int32_t reps, double* part_ms) {
       CK(cudaEventRecord(ev[0], st));
       WriteBack wb{d.v, d.qk, d.q, h->prm.time_step, h->fp32 ? 1 : 0};
       if (d.dense) {  // one launch: the first part
-        if (h->fp32)
-          launch_solve<float>(h, d.b32, d.y32, d.x32, d.Wf32, d.Wb32, 1);
-        else
-          launch_solve<double>(h, d.b64, d.y64, d.x64, d.Wf64, d.Wb64, 0);
+        launch_solve<double>(h, d.b64, d.y64, d.x64, d.Wf64, d.Wb64, 0);
         for (int k = 1; k < 5; ++k) CK(cudaEventRecord(ev[k], st));
       } else if (h->fp32)
         launch_solve_sweeps<float>(st, d.plan, d.Wf32, d.Wb32, d.b32, d.y32, d.x32, N, d.sync, wb, ev + 1);

@@ -15,19 +15,9 @@
 
 namespace pdfb {
 
-__device__ __forceinline__ float ldv(const float* p) { return __ldcg(p); }
-__device__ __forceinline__ double ldv(const double* p) { return __ldcg(p); }
-
 // 16 bytes of the inverse, and the dot products with as many entries of b
-__device__ __forceinline__ float4 ld16(const float* p) { return __ldcg(reinterpret_cast<const float4*>(p)); }
+constexpr int kVec = 2;
 __device__ __forceinline__ double2 ld16(const double* p) { return __ldcg(reinterpret_cast<const double2*>(p)); }
-__device__ __forceinline__ void dot16(float4 w, const float* b, float& s0, float& s1) {
-  const float4 v = *reinterpret_cast<const float4*>(b);
-  s0 += w.x * v.x;
-  s1 += w.y * v.y;
-  s0 += w.z * v.z;
-  s1 += w.w * v.w;
-}
 __device__ __forceinline__ void dot16(double2 w, const double* b, double& s0, double& s1) {
   const double2 v = *reinterpret_cast<const double2*>(b);
   s0 += w.x * v.x;
@@ -40,50 +30,50 @@ __device__ __forceinline__ void dot16(double2 w, const double* b, double& s0, do
 // Bound by the launch and a few memory latencies for cloths of some hundred
 // vertices (30 x 30: 6.5 MB that stay in L2), by L2 bandwidth at the limit of
 // kDenseBytes.  The solve alone, events around it, sweeps in brackets: 30 x 30
-// FP64 10 us (33), FP32 12 us (32); 53 x 53 FP64 25 us (45), 61 x 61 FP32 20 us
-// (46).
+// 10 us (33), 53 x 53 25 us (45).
+//
+// FP64 solves only.  An inverse kept in FP32 rounds each of its entries, and
+// nothing of that averages out over the rows as the sweeps' roundings do: v of
+// small cloths on a sphere was two to four times as far from the FP64 solve's as
+// with the FP32 sweeps (43 x 43: 2.5e-8 relative against 7e-9).
 constexpr int kDenseUnroll = 4;
-template <typename T>
 __global__ void __launch_bounds__(512, 2)
-    k_dense_solve(const DenseRow* __restrict__ rows, const T* __restrict__ A, const T* __restrict__ b, int n, int np,
+    k_dense_solve(const DenseRow* __restrict__ rows, const double* __restrict__ A, const double* __restrict__ b, int n, int np,
                   const int* __restrict__ perm, WriteBack wb, DTrace trace) {
   trace_stamp(trace, DTrace::kSolve);
-  constexpr int kVec = 16 / (int)sizeof(T);
-  extern __shared__ __align__(16) unsigned char smem[];
-  T* sb = reinterpret_cast<T*>(smem);
+  extern __shared__ __align__(16) double sb[];
   const int lane = threadIdx.x & 31;
   const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   // what the row needs besides b, in flight while b is staged
   DenseRow R{};
-  double qv = 0., vv = 0.;
+  double qv = 0.;
   int64_t d = 0;
   if (r < n) {
     R = rows[r];
     if (lane < 3) {
       d = 3 * (int64_t)perm[r] + lane;
       qv = wb.q[d];
-      if (wb.mode == 1) vv = wb.v[d];
     }
   }
   if (np == n) {  // one component, nothing between the planes
-    for (int k = threadIdx.x; k < 3 * n; k += blockDim.x) sb[k] = ldv(b + k);
+    for (int k = threadIdx.x; k < 3 * n; k += blockDim.x) sb[k] = __ldcg(b + k);
   } else {
-    for (int k = threadIdx.x; k < 3 * np; k += blockDim.x) sb[k] = T(0);
+    for (int k = threadIdx.x; k < 3 * np; k += blockDim.x) sb[k] = 0.;
     __syncthreads();
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
       const int at = k + rows[k].shift;
-      for (int c = 0; c < 3; ++c) sb[at + c * np] = ldv(b + k + (int64_t)c * n);
+      for (int c = 0; c < 3; ++c) sb[at + c * np] = __ldcg(b + k + (int64_t)c * n);
     }
   }
   __syncthreads();
   if (r >= n) return;
   const int ld = (R.n + kVec - 1) / kVec * kVec;
-  const T* a = A + R.off;
-  const T* bx = sb + R.c0 + R.shift;
-  T s[3][2] = {};
+  const double* a = A + R.off;
+  const double* bx = sb + R.c0 + R.shift;
+  double s[3][2] = {};
   int j = kVec * lane;
   for (; j + 32 * kVec * (kDenseUnroll - 1) < ld; j += 32 * kVec * kDenseUnroll) {
-    decltype(ld16(a)) w[kDenseUnroll];
+    double2 w[kDenseUnroll];
 #pragma unroll
     for (int u = 0; u < kDenseUnroll; ++u) w[u] = ld16(a + j + 32 * kVec * u);
 #pragma unroll
@@ -92,11 +82,11 @@ __global__ void __launch_bounds__(512, 2)
       for (int c = 0; c < 3; ++c) dot16(w[u], bx + j + 32 * kVec * u + c * np, s[c][0], s[c][1]);
   }
   for (; j < ld; j += 32 * kVec) {
-    const auto w = ld16(a + j);
+    const double2 w = ld16(a + j);
 #pragma unroll
     for (int c = 0; c < 3; ++c) dot16(w, bx + j + c * np, s[c][0], s[c][1]);
   }
-  T x[3];
+  double x[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     x[c] = s[c][0] + s[c][1];
@@ -104,27 +94,22 @@ __global__ void __launch_bounds__(512, 2)
     for (int o = 16; o > 0; o >>= 1) x[c] += __shfl_xor_sync(0xffffffffu, x[c], o);
   }
   if (lane < 3) {
-    const double val = (double)(lane == 0 ? x[0] : lane == 1 ? x[1] : x[2]) + vv;
+    const double val = lane == 0 ? x[0] : lane == 1 ? x[1] : x[2];
     wb.v[d] = val;
     wb.qk[d] = qv + wb.dt * val;
   }
 }
 
-template <typename T>
-bool launch_dense_solve(cudaStream_t st, const DenseRow* rows, const T* A, const T* b, int n, int np,
+bool launch_dense_solve(cudaStream_t st, const DenseRow* rows, const double* A, const double* b, int n, int np,
                         const int* perm, WriteBack wb, DTrace trace) {
-  const size_t smem = 3 * (size_t)np * sizeof(T);
-  if (cudaFuncSetAttribute(k_dense_solve<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmem) != cudaSuccess)
+  const size_t smem = 3 * (size_t)np * sizeof(double);
+  if (cudaFuncSetAttribute(k_dense_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, kDenseSmem) != cudaSuccess)
     return false;
   // the CTAs of all rows resident at once, on as many SMs as there are
   const int warps = std::max(4, std::min(16, (n + 147) / 148));
-  k_dense_solve<T><<<(n + warps - 1) / warps, 32 * warps, smem, st>>>(rows, A, b, n, np, perm, wb, trace);
+  k_dense_solve<<<(n + warps - 1) / warps, 32 * warps, smem, st>>>(rows, A, b, n, np, perm, wb, trace);
   return true;
 }
-template bool launch_dense_solve<double>(cudaStream_t, const DenseRow*, const double*, const double*, int, int,
-                                         const int*, WriteBack, DTrace);
-template bool launch_dense_solve<float>(cudaStream_t, const DenseRow*, const float*, const float*, int, int,
-                                        const int*, WriteBack, DTrace);
 
 // Building the inverse: the right-hand sides e_k, e_k+1, e_k+2 of every
 // component at once (k = *column), and their solutions v (vertex order) as rows
@@ -134,14 +119,13 @@ __global__ void k_dense_unit(const DenseRow* __restrict__ rows, double* __restri
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     for (int c = 0; c < 3; ++c) b[i + (int64_t)c * n] = i - rows[i].c0 == k + c ? 1. : 0.;
 }
-template <typename T>
 __global__ void k_dense_rows(const DenseRow* __restrict__ rows, const double* __restrict__ v, int n,
-                             const int* __restrict__ perm, T* __restrict__ A, const int* column) {
+                             const int* __restrict__ perm, double* __restrict__ A, const int* column) {
   const int k = *column;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const int c0 = rows[i].c0;
     for (int c = 0; c < 3; ++c)
-      if (k + c < rows[i].n) A[rows[c0 + k + c].off + i - c0] = (T)v[3 * (int64_t)perm[i] + c];
+      if (k + c < rows[i].n) A[rows[c0 + k + c].off + i - c0] = v[3 * (int64_t)perm[i] + c];
   }
 }
 __global__ void k_dense_next(int* column, int step) { *column += step; }
@@ -149,14 +133,10 @@ __global__ void k_dense_next(int* column, int step) { *column += step; }
 void launch_dense_unit(cudaStream_t st, const DenseRow* rows, double* b, int n, const int* column) {
   k_dense_unit<<<std::min(148, (n + 255) / 256), 256, 0, st>>>(rows, b, n, column);
 }
-template <typename T>
-void launch_dense_rows(cudaStream_t st, const DenseRow* rows, const double* v, int n, const int* perm, T* A,
+void launch_dense_rows(cudaStream_t st, const DenseRow* rows, const double* v, int n, const int* perm, double* A,
                        int* column, int step) {
-  k_dense_rows<T><<<std::min(148, (n + 255) / 256), 256, 0, st>>>(rows, v, n, perm, A, column);
+  k_dense_rows<<<std::min(148, (n + 255) / 256), 256, 0, st>>>(rows, v, n, perm, A, column);
   k_dense_next<<<1, 1, 0, st>>>(column, step);
 }
-template void launch_dense_rows<double>(cudaStream_t, const DenseRow*, const double*, int, const int*, double*, int*,
-                                        int);
-template void launch_dense_rows<float>(cudaStream_t, const DenseRow*, const double*, int, const int*, float*, int*, int);
 
 }  // namespace pdfb

@@ -226,8 +226,7 @@ bool blocked_cholesky(double* F, int ns, int ld) {
 
 }  // namespace
 
-bool factorize(const Model& m, double dt, int leaf_size, Factor& f, std::string& err,
-               bool (*apart)(const std::vector<int>& sizes)) {
+bool factorize(const Model& m, double dt, int leaf_size, Factor& f, std::string& err, bool fp32) {
   auto t_start = std::chrono::steady_clock::now();
   const int N = m.N;
   f.N = N;
@@ -238,14 +237,12 @@ bool factorize(const Model& m, double dt, int leaf_size, Factor& f, std::string&
     // batch) on its own: dissected together, components that overlap in space
     // share supernodes, whose dense blocks hold a zero for every pair of rows of
     // different components (three 128 x 128 layers: 16.5 M stored entries against 6.1 M).
-    // FP32 sweeps (`apart`) keep layers together: apart, their result was further
+    // FP32 sweeps keep layers together: apart, their result was further
     // from the FP64 solve's by a fifth (two 256 x 256 layers, one step of 20
     // iterations, six inputs: 2.2e-6 to 2.4e-6
     // relative against 2.0e-6), for all that a solve took 0.105 ms instead of 0.136
     std::vector<std::vector<int>> comps = components(m);
-    std::vector<int> sizes;
-    for (const std::vector<int>& ids : comps) sizes.push_back((int)ids.size());
-    if (apart && comps.size() > 1 && !apart(sizes)) comps = united(m, comps);
+    if (fp32 && comps.size() > 1) comps = united(m, comps);
     for (std::vector<int>& ids : comps) {
       f.comp_ptr.push_back((int)nd.order.size());
       nd.run(ids);

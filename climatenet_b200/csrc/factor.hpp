@@ -70,10 +70,9 @@ struct Factor {
 };
 
 // Returns false (and sets err) if the matrix is not positive definite.
-// Components are dissected one by one; where `apart` is given and refuses their
-// sizes, those that overlap in space are dissected together (factorize).
-bool factorize(const Model& m, double dt, int leaf_size, Factor& f, std::string& err,
-               bool (*apart)(const std::vector<int>& sizes) = nullptr);
+// Components are dissected one by one; for FP32 sweeps those that overlap in
+// space are dissected together (factorize).
+bool factorize(const Model& m, double dt, int leaf_size, Factor& f, std::string& err, bool fp32 = false);
 
 // One warp's work item of a supernodal sweep: tile `tile` of supernode `sn`
 // (rows 32 tile.. of W_s for the forward sweep, columns for the backward one),

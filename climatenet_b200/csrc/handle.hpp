@@ -42,11 +42,10 @@ struct DeviceBuffers {
   SweepSync sync{};
   double *b64 = nullptr, *y64 = nullptr, *x64 = nullptr;
   float *b32 = nullptr, *y32 = nullptr, *x32 = nullptr;
-  // small scenes: the explicit inverse, in the solve's precision
+  // small FP64 scenes: the explicit inverse
   DenseRow* dense_rows = nullptr;
   int dense_np = 0;  // columns with each component padded to 16 bytes
-  double* dense64 = nullptr;
-  float* dense32 = nullptr;
+  double* inverse = nullptr;
   bool dense = false;  // it is what solves (pdf_set_sweep_schedule turns to the sweeps)
   // contacts
   DContacts c{};

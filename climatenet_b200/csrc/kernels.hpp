@@ -203,15 +203,14 @@ void launch_solve_sweeps(cudaStream_t st, const DPlan& P, const T* Wf, const T* 
 template <typename T>
 void launch_solve_prep(cudaStream_t st, int n, T* x, T* y, SweepSync sy);
 
-// Small scenes: the solve as one product with the explicit inverse
+// Small FP64 scenes: the solve as one product with the explicit inverse
 // (dense_solve.cu).  The inverse is kept where it takes at most kDenseBytes and
 // b fits the kernel's shared memory (two CTAs an SM).  Below the limit the product
-// reads L2-resident rows and beats the sweeps' chain of launches (30 x 30 FP64:
-// 6.5 MB, 10 us against 33; at the limit, 64 x 64 FP32: 23 us against 47); above
+// reads L2-resident rows and beats the sweeps' chain of launches (30 x 30:
+// 6.5 MB, 10 us against 33; near the limit, 53 x 53: 25 us against 45); above
 // it the inverse grows with N^2 where the factor grows with N log N, and leaves L2.
 // Its construction (a third of N solves) replaces the schedule autotuner there:
-// creating a 30 x 30 cloth takes 13 ms (28 before), a 61 x 61 FP32 one 38 ms
-// (45 before).
+// creating a 30 x 30 cloth takes 13 ms (28 before).
 constexpr size_t kDenseBytes = size_t(64) << 20;
 constexpr int kDenseSmem = 100 * 1024;
 struct DenseRow {
@@ -219,12 +218,10 @@ struct DenseRow {
   int c0, n;    // its component: first column, columns
   int shift;    // c0 + shift is where the component's entries start in a padded plane
 };
-template <typename T>
-bool launch_dense_solve(cudaStream_t st, const DenseRow* rows, const T* A, const T* b, int n, int np,
+bool launch_dense_solve(cudaStream_t st, const DenseRow* rows, const double* A, const double* b, int n, int np,
                         const int* perm, WriteBack wb, DTrace trace);  // np: entries of a padded plane
 void launch_dense_unit(cudaStream_t st, const DenseRow* rows, double* b, int n, const int* column);
-template <typename T>
-void launch_dense_rows(cudaStream_t st, const DenseRow* rows, const double* v, int n, const int* perm, T* A,
+void launch_dense_rows(cudaStream_t st, const DenseRow* rows, const double* v, int n, const int* perm, double* A,
                        int* column, int step);  // then *column += step
 
 // detection (detect_kernels.cu, compiled without FMA contraction)
