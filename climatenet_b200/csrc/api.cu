@@ -692,9 +692,12 @@ bool build_dense(pdf_handle* h) {
 // kernels at 2 CTAs of 8 or 4 CTAs of 4 consumer warps per SM where they
 // fit; dependency-driven upper items, the slower mode, only where the levels do
 // not fit the launch table), then with each launch shape of the block kernels at the best cut
-// level and mode, then with each work-item width, and keeps the fastest.  The right-hand side is
-// zero (the sweeps read the same data and wait on the same dependencies
-// whatever the values); v and q^k, which the solve writes, are restored.
+// level and mode, then, in FP64, with each work-item width, and keeps the fastest.  (The
+// width groups the sums: FP32 results would take over the timing's choice.  Two
+// 256 x 256 layers: v with 64-column items and two chains a sum was 1.26 times as far
+// from a run with 32 as two such runs from each other; now 1.05 times.)
+// The right-hand side is zero (the sweeps read the same data and wait on the same
+// dependencies whatever the values); v and q^k, which the solve writes, are restored.
 void autotune_schedule(pdf_handle* h) {
   DeviceBuffers& d = h->d;
   const int N = h->dm.N;
@@ -773,6 +776,7 @@ void autotune_schedule(pdf_handle* h) {
   const double best_default_chunk = best;
   for (int ci = 0; ci < 3; ++ci) {
     const int chunk = kChunkCandidates[ci];
+    if (h->fp32 && chunk != kChunk) continue;
     const double ms =
         chunk == kChunk ? best_default_chunk : time_plan(chunk, best_cut, best_mode, best_shape, true);
     h->stats.sweep_chunk_ms[ci] = ms;

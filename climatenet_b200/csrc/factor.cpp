@@ -181,16 +181,18 @@ std::vector<std::vector<int>> united(const Model& m, const std::vector<std::vect
 // Top dissection levels merged into the root supernode (PDF_ND_MERGE
 // overrides it for tuning experiments).  A merged level saves a launch per sweep
 // (some 3 us each) and fills the root: by 40 N entries from three levels to four, by
-// 24 N from two to three, N the scene's vertices.  Solves measured in FP64, FP32
-// alike: 9.4k vertices 49 us at 3, 42 at 4 (5: 39, but the root's factorisation
-// takes 100 ms instead of 24); 15.6k 54 and 49; 22.5k 61 and 59; 40k 72 and 73;
-// 250k 234 at 3, 230 at 2.
-int nd_merge_levels(int N) {
+// 24 N from two to three, N the scene's vertices.  FP64 solves: 9.4k vertices 49 us
+// at 3, 42 at 4 (5: 39, but the root's factorisation takes 100 ms instead of 24);
+// 15.6k 54 and 49; 22.5k 61 and 59; 40k 72 and 73; 250k 234 at 3, 230 at 2.
+// FP32 sweeps have three at every size: another factor rounds otherwise, and on small
+// cloths the roundings of the factor are most of what v differs by (24 x 24 on a
+// floor: twice as far from a run with three levels as two such runs are apart).
+int nd_merge_levels(int N, bool fp32) {
   if (const char* e = std::getenv("PDF_ND_MERGE")) {
     const int v = std::atoi(e);
     if (v >= 0 && v <= 16) return v;
   }
-  return N <= 20000 ? 4 : N <= 200000 ? 3 : 2;
+  return fp32 ? 3 : N <= 20000 ? 4 : N <= 200000 ? 3 : 2;
 }
 
 // In-place Cholesky of the leading ns x ns block of the row-major front F
@@ -231,7 +233,7 @@ bool factorize(const Model& m, double dt, int leaf_size, Factor& f, std::string&
   const int N = m.N;
   f.N = N;
   // ---- ordering and supernode partition -------------------------------
-  NDBuilder nd(m, std::max(8, leaf_size), nd_merge_levels(N));
+  NDBuilder nd(m, std::max(8, leaf_size), nd_merge_levels(N, fp32));
   {
     // each connected component of the matrix graph (a layer, a cloth of a
     // batch) on its own: dissected together, components that overlap in space

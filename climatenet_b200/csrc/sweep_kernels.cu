@@ -1033,7 +1033,10 @@ __global__ void __launch_bounds__(32 * kLevelWarps)
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
             fma_vec(vs + 4 * j, w[m * j], ax, ay, az);
-            fma_vec(vs + 4 * j + 4, w[m * j + m], bx, by, bz);
+            if (sizeof(T) == 4)  // FP32 sums in column order, as the blocks'
+              fma_vec(vs + 4 * j + 4, w[m * j + m], ax, ay, az);
+            else
+              fma_vec(vs + 4 * j + 4, w[m * j + m], bx, by, bz);
           }
         } else {
 #pragma unroll 8
