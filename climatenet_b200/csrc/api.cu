@@ -508,7 +508,7 @@ void create_impl(pdf_handle* h, const pdf_scene_desc* sc, const pdf_params* p) {
     d.cub_tmp = dalloc<char>(d.cub_tmp_bytes);
   }
   if (p->self_collision) {
-    CK(configure_friction_self());
+    h->self_ctas = friction_self_ctas();
     int st = self_detect_init(h);
     if (st != PDF_OK) throw CudaFail("self-collision workspace: " + h->err);
   }
@@ -810,7 +810,7 @@ void launch_iteration(pdf_handle* h, T* b, T* y, T* x, const T* Wf, const T* Wb,
   const bool warm = h->prm.warm_start == PDF_WARM_MLP;
   launch_friction_obstacle<T>(kStrideBlocks, kThreads, st, dm, d.c, b, self_mode, d.iter, warm ? h->mlp_Y : nullptr,
                               warm ? gravity_dt(h) : 0.);
-  if (self_mode) launch_friction_self<T>(st, dm, d.c, b, d.newf, d.iter);
+  if (self_mode) CK(launch_friction_self<T>(st, h->self_ctas, dm, d.c, b, d.newf, d.iter));
   launch_solve<T>(h, b, y, x, Wf, Wb, mode);
   IterCtl ctl{d.iter, d.iter_total, d.blocks_done, h->prm.residual_tolerance, h->prm.local_global_iterations,
               h->capturing_cond ? 1 : 0, h->cond, h->dm.trace};

@@ -117,6 +117,7 @@ struct pdf_handle {
   cudaGraphExec_t graph = nullptr;
   int graph_iters = 0;
   int n_levels = 0;
+  int self_ctas = 1;  // of the self-friction kernel's cluster
   int cap_contacts = 0, cap_self = 0;
   double time = 0.;
   std::string err;

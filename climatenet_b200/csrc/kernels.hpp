@@ -188,8 +188,9 @@ template <typename T>
 void launch_friction_obstacle(dim3 grid, dim3 block, cudaStream_t st, DModel m, DContacts c, T* b, int self_mode,
                               const int* iter, const float* pred = nullptr, double pred_sv = 0.);
 template <typename T>
-void launch_friction_self(cudaStream_t st, DModel m, DContacts c, T* b, double* newf, const int* iter);
-cudaError_t configure_friction_self();  // before its first launch on a device
+cudaError_t launch_friction_self(cudaStream_t st, int ctas, DModel m, DContacts c, T* b, double* newf,
+                                 const int* iter);
+int friction_self_ctas();  // ctas for the current device
 // Solve vectors b, y, x are three planes of n values (x, y, z components) in
 // pivot order.  y and x of the upper supernodes must be zero before a solve
 // (the previous solve's backward and this one's forward block kernel see to

@@ -5,6 +5,9 @@
 // project root ("SFE" = src/physics/SimulationFrictionEstimation.cpp).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cstdlib>
+
 #include "device.cuh"
 #include "kernels.hpp"
 
@@ -490,29 +493,51 @@ __global__ void __launch_bounds__(kSelfThreads)
     st3(c.sf[cur], s, make_double3(0., 0., 0.));
   }
 }
-template <typename T>
-void launch_friction_self(cudaStream_t st, DModel m, DContacts c, T* b, double* newf, const int* iter) {
+inline cudaLaunchConfig_t self_config(int ctas, cudaLaunchAttribute* attr, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(kSelfCtas);
+  cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(kSelfThreads);
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = kSelfCtas;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = ctas;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k_friction_self<T>, m, c, b, newf, iter);
+  return cfg;
 }
-// Clusters of more than 8 CTAs are opt-in, once per process and device.
-cudaError_t configure_friction_self() {
-  cudaError_t e = cudaFuncSetAttribute(k_friction_self<double>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_friction_self<float>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  return e;
+template <typename T>
+cudaError_t launch_friction_self(cudaStream_t st, int ctas, DModel m, DContacts c, T* b, double* newf,
+                                 const int* iter) {
+  cudaLaunchAttribute attr[1];
+  const cudaLaunchConfig_t cfg = self_config(ctas, attr, st);
+  return cudaLaunchKernelEx(&cfg, k_friction_self<T>, m, c, b, newf, iter);
 }
-template void launch_friction_self<double>(cudaStream_t, DModel, DContacts, double*, double*, const int*);
-template void launch_friction_self<float>(cudaStream_t, DModel, DContacts, float*, double*, const int*);
+// The CTAs of the cluster: the most, up to kSelfCtas, that the device can host
+// together (a part of a GPU may have no 16 SMs that form one); one always runs.
+// PDF_SELF_CTAS lowers the limit.
+int friction_self_ctas() {
+  int most = kSelfCtas;
+  if (const char* e = std::getenv("PDF_SELF_CTAS")) most = std::max(1, std::min(kSelfCtas, std::atoi(e)));
+  for (int ctas = kSelfCtas; ctas > 1; ctas /= 2) {
+    if (ctas > most) continue;
+    // more than 8 are opt-in, once per process and device
+    bool fits = ctas <= 8 ||
+                (cudaFuncSetAttribute(k_friction_self<double>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                     cudaSuccess &&
+                 cudaFuncSetAttribute(k_friction_self<float>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                     cudaSuccess);
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg = self_config(ctas, attr, 0);
+    int n64 = 0, n32 = 0;
+    fits = fits && cudaOccupancyMaxActiveClusters(&n64, k_friction_self<double>, &cfg) == cudaSuccess && n64 > 0 &&
+           cudaOccupancyMaxActiveClusters(&n32, k_friction_self<float>, &cfg) == cudaSuccess && n32 > 0;
+    cudaGetLastError();
+    if (fits) return ctas;
+  }
+  return 1;
+}
+template cudaError_t launch_friction_self<double>(cudaStream_t, int, DModel, DContacts, double*, double*, const int*);
+template cudaError_t launch_friction_self<float>(cudaStream_t, int, DModel, DContacts, float*, double*, const int*);
 
 // Alart-Curnier residual with rho = 1 (coulomb_util.cpp:92-152) for every
 // contact after the solve (SFE:590-652).  acc[4] += {sum |AC|, max |AC|,
