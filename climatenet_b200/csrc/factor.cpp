@@ -131,6 +131,28 @@ std::vector<std::vector<int>> components(const Model& m) {
   return out;
 }
 
+// Components of up to `leaf` vertices in all, gathered in their order: a block of the
+// sweeps costs its CTA some 5 us, whatever it holds.  20,000 cloths of 3 x 3, a step of
+// 20 iterations in FP64: 6.7 ms with a block each, 3.2 ms gathered, 4.1 ms in one
+// dissection; 60,000 of 2 x 2: 16.8, 3.3 and 4.6 ms.
+std::vector<std::vector<int>> gathered(std::vector<std::vector<int>> comps, int leaf) {
+  std::vector<std::vector<int>> out;
+  std::vector<int> small;
+  for (std::vector<int>& ids : comps) {
+    if ((int)ids.size() > leaf) {
+      out.push_back(std::move(ids));
+      continue;
+    }
+    if ((int)(small.size() + ids.size()) > leaf) {
+      out.push_back(std::move(small));
+      small.clear();
+    }
+    small.insert(small.end(), ids.begin(), ids.end());
+  }
+  if (!small.empty()) out.push_back(std::move(small));
+  return out;
+}
+
 // The components whose bounding boxes overlap (layers) united, vertices ascending.
 std::vector<std::vector<int>> united(const Model& m, const std::vector<std::vector<int>>& comps) {
   const int n = (int)comps.size();
@@ -143,17 +165,34 @@ std::vector<std::vector<int>> united(const Model& m, const std::vector<std::vect
         box[c][3 + k] = std::max(box[c][3 + k], m.rest[3 * (size_t)v + k]);
       }
   }
-  std::vector<int> set(n), by_x(n);
+  // pairs are looked for along the axis in which the boxes overlap least
+  int ax = 0;
+  double least = 1e300, reach = 0.;  // no pair further apart than `reach` is united
+  for (int k = 0; k < 3; ++k) {
+    double lo = 1e300, hi = -1e300, sum = 0.;
+    for (const auto& b : box) {
+      lo = std::min(lo, b[k]);
+      hi = std::max(hi, b[3 + k]);
+      sum += b[3 + k] - b[k];
+      reach = std::max(reach, 0.05 * (b[3 + k] - b[k]));
+    }
+    if (hi > lo && sum / (hi - lo) < least) {
+      least = sum / (hi - lo);
+      ax = k;
+    }
+  }
+  std::vector<int> set(n), by_ax(n);
   std::iota(set.begin(), set.end(), 0);
-  std::iota(by_x.begin(), by_x.end(), 0);
+  std::iota(by_ax.begin(), by_ax.end(), 0);
   auto root = [&](int c) {
     while (set[c] != c) c = set[c] = set[set[c]];
     return c;
   };
-  std::sort(by_x.begin(), by_x.end(), [&](int a, int b) { return box[a][0] < box[b][0]; });
+  std::sort(by_ax.begin(), by_ax.end(), [&](int a, int b) { return box[a][ax] < box[b][ax]; });
   for (int i = 0; i < n; ++i)
-    for (int j = i + 1; j < n && box[by_x[j]][0] <= box[by_x[i]][3]; ++j) {
-      const auto &a = box[by_x[i]], &b = box[by_x[j]];
+    for (int j = i + 1; j < n && box[by_ax[j]][ax] <= box[by_ax[i]][3 + ax] + reach; ++j) {
+      const auto &a = box[by_ax[i]], &b = box[by_ax[j]];
+      if (a[0] > b[3] || b[0] > a[3]) continue;
       // in the plane of the two widest extents layers cover each other; along the
       // third they may lie apart
       int over = 0;
@@ -164,7 +203,7 @@ std::vector<std::vector<int>> united(const Model& m, const std::vector<std::vect
         side = std::max(side, std::min(a[3 + k] - a[k], b[3 + k] - b[k]));
       }
       if (over == 3 || (over == 2 && gap < 0.05 * side)) {
-        const int ra = root(by_x[i]), rb = root(by_x[j]);
+        const int ra = root(by_ax[i]), rb = root(by_ax[j]);
         set[std::max(ra, rb)] = std::min(ra, rb);
       }
     }
@@ -236,14 +275,14 @@ bool factorize(const Model& m, double dt, int leaf_size, Factor& f, std::string&
   NDBuilder nd(m, std::max(8, leaf_size), nd_merge_levels(N, fp32));
   {
     // each connected component of the matrix graph (a layer, a cloth of a
-    // batch) on its own: dissected together, components that overlap in space
+    // batch; the smallest gathered) on its own: dissected together, components that overlap in space
     // share supernodes, whose dense blocks hold a zero for every pair of rows of
     // different components (three 128 x 128 layers: 16.5 M stored entries against 6.1 M).
     // FP32 sweeps keep layers together: apart, their result was further
     // from the FP64 solve's by a fifth (two 256 x 256 layers, one step of 20
     // iterations, six inputs: 2.2e-6 to 2.4e-6
     // relative against 2.0e-6), for all that a solve took 0.105 ms instead of 0.136
-    std::vector<std::vector<int>> comps = components(m);
+    std::vector<std::vector<int>> comps = gathered(components(m), std::max(8, leaf_size));
     if (fp32 && comps.size() > 1) comps = united(m, comps);
     for (std::vector<int>& ids : comps) {
       f.comp_ptr.push_back((int)nd.order.size());

@@ -61,7 +61,7 @@ struct Factor {
   std::vector<int64_t> sn_ftile0, sn_btile0;
   std::vector<int64_t> ftile_off, btile_off;  // per tile, +1 sentinel
   std::vector<double> Wf, Wb;
-  std::vector<int> comp_ptr;     // connected components: columns [comp_ptr[c], comp_ptr[c + 1])
+  std::vector<int> comp_ptr;     // connected components (or sets of them): columns [comp_ptr[c], comp_ptr[c + 1])
   int n_levels = 0;
   int64_t nnz_w = 0;             // sum ns(ns+1)/2 + nr ns
   int64_t nnz_l_true = 0;        // structural nnz of L (diagonal included)
@@ -70,8 +70,8 @@ struct Factor {
 };
 
 // Returns false (and sets err) if the matrix is not positive definite.
-// Components are dissected one by one; for FP32 sweeps those that overlap in
-// space are dissected together (factorize).
+// Components are dissected one by one, the smallest gathered; for FP32 sweeps
+// those that overlap in space are dissected together (factorize).
 bool factorize(const Model& m, double dt, int leaf_size, Factor& f, std::string& err, bool fp32 = false);
 
 // One warp's work item of a supernodal sweep: tile `tile` of supernode `sn`
