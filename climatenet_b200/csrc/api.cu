@@ -588,7 +588,8 @@ void launch_solve_with(pdf_handle* h, const SweepSync& sy, T* b, T* y, T* x, con
 
 // Small FP64 scenes (kDenseBytes): the explicit inverse, its columns three at a
 // time by the sweeps, a captured set of solves replayed.  false where the scene is
-// too large, or memory too short.
+// too large, or where there is no memory for the inverse or for building it: the
+// sweeps solve then.  (PDF_DENSE_ROOM=k: the memory ends after k allocations.)
 bool build_dense(pdf_handle* h) {
   DeviceBuffers& d = h->d;
   const Factor& f = h->fac;
@@ -606,24 +607,35 @@ bool build_dense(pdf_handle* h) {
     total += (int64_t)n * ld;
     widest = std::max(widest, n);
   }
-  d.dense_np = (int)np;
+  // leaves and their parents as blocks, 32-column items by level (solves side by
+  // side must not share the counters of the dependency-driven mode), 2 CTAs of 8 warps
+  build_schedule(h, 32, 1, 1, 1);
+  if (d.plan.upper_mode != 1) return false;
   cudaStream_t st = h->stream;
-  void* mem = nullptr;
-  if (cudaMalloc(&mem, total * sizeof(double)) != cudaSuccess) {  // no room for it: the sweeps
-    cudaGetLastError();
-    return false;
-  }
-  d.inverse = (double*)mem;
-  d.dense_rows = upload(rows);
-  CK(cudaMemsetAsync(d.inverse, 0, total * sizeof(double), st));  // the rows' padding
   // kBranches sweeps side by side (each is a chain of short launches): vectors,
   // queues, solve counter and column of their own
   constexpr int kBranches = 4;
+  struct NoRoom {};
+  auto need = [](cudaError_t e) {
+    if (e == cudaErrorMemoryAllocation) throw NoRoom{};
+    CK(e);
+  };
+  const char* limit = std::getenv("PDF_DENSE_ROOM");
+  int left = limit ? std::atoi(limit) : -1;
   std::vector<void*> tmp;
+  auto get = [&](size_t bytes) {
+    if (left == 0) throw NoRoom{};
+    if (left > 0) --left;
+    void* p = nullptr;
+    need(cudaMalloc(&p, bytes));
+    tmp.push_back(p);
+    return p;
+  };
   cudaStream_t side[kBranches] = {};
   cudaEvent_t ev[kBranches] = {};
   cudaGraphExec_t exec = nullptr;
   auto release = [&] {
+    cudaStreamSynchronize(st);
     if (exec) cudaGraphExecDestroy(exec);
     for (void* p : tmp) cudaFree(p);
     for (cudaStream_t s2 : side)
@@ -631,26 +643,30 @@ bool build_dense(pdf_handle* h) {
     for (cudaEvent_t e2 : ev)
       if (e2) cudaEventDestroy(e2);
   };
+  double* inverse = nullptr;
+  DenseRow* drows = nullptr;
   try {
-    // leaves and their parents as blocks, 32-column items, 2 CTAs of 8 warps
-    build_schedule(h, 32, 1, 1, 1);
+    inverse = (double*)get(total * sizeof(double));
+    drows = (DenseRow*)get(rows.size() * sizeof(DenseRow));
+    CK(cudaMemcpy(drows, rows.data(), rows.size() * sizeof(DenseRow), cudaMemcpyHostToDevice));
+    CK(cudaMemsetAsync(inverse, 0, total * sizeof(double), st));  // the rows' padding
     double* vec[kBranches];  // b, y, x, v, q^k
     int* column[kBranches];
     SweepSync sy[kBranches];
     const size_t n3 = 3 * (size_t)N;
     for (int k = 0; k < kBranches; ++k) {
-      tmp.push_back(vec[k] = dalloc<double>(5 * n3));
-      tmp.push_back(column[k] = dalloc<int>(1));
+      vec[k] = (double*)get(5 * n3 * sizeof(double));
+      column[k] = (int*)get(sizeof(int));
       const int first = 3 * k;
       CK(cudaMemcpyAsync(column[k], &first, sizeof(int), cudaMemcpyHostToDevice, st));
       sy[k] = d.sync;
       sy[k].trace.stamps = nullptr;
-      tmp.push_back(sy[k].queue = dalloc<int>(4));
-      tmp.push_back(sy[k].epoch = dalloc<unsigned long long>(1));
+      sy[k].queue = (int*)get(4 * sizeof(int));
+      sy[k].epoch = (unsigned long long*)get(sizeof(unsigned long long));
       CK(cudaMemsetAsync(sy[k].epoch, 0, sizeof(unsigned long long), st));
       launch_solve_prep<double>(st, N, vec[k] + 2 * n3, vec[k] + n3, sy[k]);
-      CK(cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming));
-      if (k > 0) CK(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking));
+      need(cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming));
+      if (k > 0) need(cudaStreamCreateWithFlags(&side[k], cudaStreamNonBlocking));
     }
     cudaGraph_t g;
     CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -659,27 +675,34 @@ bool build_dense(pdf_handle* h) {
       cudaStream_t s2 = k > 0 ? side[k] : st;
       if (k > 0) cudaStreamWaitEvent(s2, ev[0], 0);
       double *b = vec[k], *y = b + n3, *x = y + n3, *v = x + n3, *qk = v + n3;
-      launch_dense_unit(s2, d.dense_rows, b, N, column[k]);
+      launch_dense_unit(s2, drows, b, N, column[k]);
       launch_solve_sweeps<double>(s2, d.plan, d.Wf64, d.Wb64, b, y, x, N, sy[k], WriteBack{v, qk, d.q, 0., 0});
-      launch_dense_rows(s2, d.dense_rows, v, N, d.perm, d.inverse, column[k], 3 * kBranches);
+      launch_dense_rows(s2, drows, v, N, d.perm, inverse, column[k], 3 * kBranches);
       if (k > 0) cudaEventRecord(ev[k], s2);
     }
     for (int k = 1; k < kBranches; ++k) cudaStreamWaitEvent(st, ev[k], 0);
     CK(cudaStreamEndCapture(st, &g));
     const cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
     cudaGraphDestroy(g);
-    CK(e);
-    for (int k = 0; k < widest; k += 3 * kBranches) CK(cudaGraphLaunch(exec, st));
+    need(e);
+    for (int k = 0; k < widest; k += 3 * kBranches) need(cudaGraphLaunch(exec, st));
     CK(cudaStreamSynchronize(st));
     int derr = 0;
     CK(cudaMemcpy(&derr, d.sync.err, sizeof(int), cudaMemcpyDeviceToHost));
     if (derr) throw CudaFail("a supernodal sweep gave up waiting while the inverse was built");
+  } catch (const NoRoom&) {
+    release();
+    cudaGetLastError();
+    return false;
   } catch (...) {
-    cudaStreamSynchronize(st);
     release();
     throw;
   }
+  tmp.erase(tmp.begin(), tmp.begin() + 2);  // the inverse and its rows stay
   release();
+  d.dense_np = (int)np;
+  d.inverse = inverse;
+  d.dense_rows = drows;
   // the schedule the sweeps would take, should pdf_set_sweep_schedule ask for them
   launch_solve_prep<double>(st, N, d.x64, d.y64, d.sync);
   CK(cudaStreamSynchronize(st));
