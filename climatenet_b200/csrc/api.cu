@@ -1299,7 +1299,14 @@ int pdf_time_phase(pdf_handle* h, int32_t phase, int32_t reps, double* ms_out, d
     const double N = dm.N;
     double bytes = 0;
     int64_t idx_rows = (int64_t)f.rows.size();
-    if (phase == 0) {
+    if (phase == 0 && d.dense) {
+      // the components' inverses, b, the permutation, write-back (q read; v, q^k written)
+      for (size_t c = 0; c + 1 < f.comp_ptr.size(); ++c) {
+        const double n = f.comp_ptr[c + 1] - f.comp_ptr[c];
+        bytes += 8. * n * n;
+      }
+      bytes += (24. + 4. + 72.) * N;
+    } else if (phase == 0) {
       // 2 [l s + idx_bytes(L)] + 2 (2 * 3 s N) + FP64 write-back (q read; v, q^k
       // written), with l = structural nnz(L) (padding and explicit zeros of the
       // stored tiles are not counted)
@@ -1315,10 +1322,10 @@ int pdf_time_phase(pdf_handle* h, int32_t phase, int32_t reps, double* ms_out, d
       // obstacle tests: positions read, one flag byte per (obstacle, vertex);
       // self collision (when on): positions and triangles read (24 N + 12 T),
       // the 112-byte node records written by the refit and read once by the
-      // traversal, and the triangle boxes (48 T) written and read
+      // traversal
       const double T = (double)h->model.tris.size() / 3.;
       bytes = (double)h->obs.n * (24. * N + N);
-      if (h->prm.self_collision) bytes += 24. * N + 12. * T + 2. * 112. * std::max(0., T - 1.) + 2. * 48. * T;
+      if (h->prm.self_collision) bytes += 24. * N + 12. * T + 2. * 112. * std::max(0., T - 1.);
     }
     // phase 0 works on a saved right-hand side restored between repetitions
     double* save64 = nullptr;

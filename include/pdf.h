@@ -360,7 +360,9 @@ int pdf_get_residual_history(pdf_handle* h, double* out, int32_t cap,
  * projection, 3 = detection (obstacles and self-collision).  The state is not
  * advanced in a meaningful way; call it before or after a measured run.
  * *bytes receives the algorithmic bytes one repetition must move (phases 0,
- * 1 and 3; 0 for phase 2). */
+ * 1 and 3; 0 for phase 2): in phase 0 the factor's entries and the vectors of
+ * both sweeps or, for scenes solved by one product with the inverse, the
+ * inverse, its right-hand side and the write-back. */
 int pdf_time_phase(pdf_handle* h, int32_t phase, int32_t reps, double* ms,
                    double* bytes);
 
