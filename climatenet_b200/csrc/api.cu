@@ -1852,7 +1852,8 @@ int pdf_factor_check(const pdf_scene_desc* scene, const pdf_params* params, cons
     build_model(*scene, *params, m);
     Factor f;
     std::string err;
-    if (!factorize(m, params->time_step, 40, f, err)) return fail(nullptr, PDF_NOT_SPD, err);
+    const bool fp32 = params->precision == PDF_FP32_REFINE;  // whose factor may be another
+    if (!factorize(m, params->time_step, 40, f, err, fp32)) return fail(nullptr, PDF_NOT_SPD, err);
     std::vector<double> bv(b, b + 3 * (size_t)m.N), xv;
     // every schedule the autotuner can choose: cut levels 0 .. 7, chunks
     // 32 / 64 / 128; all must solve the system alike
