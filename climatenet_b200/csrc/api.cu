@@ -1792,11 +1792,15 @@ int pdf_set_sweep_schedule(pdf_handle* h, int32_t chunk, int32_t cut_level, int3
   return guarded(h, [&]() -> int {
     CK(cudaSetDevice(h->prm.device));
     CK(cudaStreamSynchronize(h->stream));
-    h->d.dense = false;
     build_schedule(h, chunk, cut_level, upper_mode, block_shape);
     const bool mode_ok = h->d.plan.upper_mode == upper_mode && h->d.plan.block_shape == block_shape;
     if (!mode_ok) build_schedule(h, chunk, cut_level, 0, 0);
     DeviceBuffers& d = h->d;
+    if (mode_ok && d.dense) {  // the inverse is not needed any more
+      d.dense = false;
+      free_dev(d.inverse);
+      free_dev(d.dense_rows);
+    }
     if (h->fp32)
       launch_solve_prep<float>(h->stream, h->dm.N, d.x32, d.y32, d.sync);
     else

@@ -247,7 +247,11 @@ int pdf_params_load_json(const char* json_path, pdf_params* out,
  * (src/simulation_building.cpp:80-98) and the constructors it runs
  * (SimulationFrictionEstimation SFE:31-62, SimulationSpeed.cpp:29-60,
  * SimulationBase.cpp:46-100): assembles A, the LHS M + dt^2 A^T A, its one-time
- * Cholesky factor, and uploads everything to the device. */
+ * Cholesky factor, and uploads everything to the device.
+ * FP64 scenes of up to some 2,900 vertices (more in several components) also
+ * hold the inverse of that matrix, 8 bytes for each pair of vertices of a
+ * component and 64 MiB at the most (30 x 30: 6.5 MB); it is left out where
+ * there is no room for it, and pdf_set_sweep_schedule gives it back. */
 int pdf_create(const pdf_scene_desc* scene, const pdf_params* params,
                pdf_handle** out);
 
@@ -383,7 +387,10 @@ int pdf_time_solve_parts(pdf_handle* h, int32_t reps, double* part_ms);
  * sweep_block_shape).  Every schedule solves the same system; the results
  * agree to rounding.  PDF_INVALID_ARG for values outside these sets, for
  * mode 1 on a scene with more upper levels than the launch table holds
- * (stats sweep_upper_levels), or for a shape the blocks do not fit. */
+ * (stats sweep_upper_levels), or for a shape the blocks do not fit.  A small
+ * scene solved by one product with the inverse (pdf_create) solves by the
+ * sweeps from then on and gives the inverse's memory back; one whose schedule
+ * is refused keeps it. */
 int pdf_set_sweep_schedule(pdf_handle* h, int32_t chunk, int32_t cut_level,
                            int32_t upper_mode, int32_t block_shape);
 
