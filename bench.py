@@ -359,12 +359,12 @@ def e2e_steps(sim, steps, barrier, dist, world, start):
 
 
 # DRAM bytes (read + write) of one global solve of the 500 x 500 cloth, all
-# launches of the forward and backward sweeps and the write-back, summed from
+# launches of the forward and backward sweeps, summed from
 # ncu's dram__bytes_read.sum + dram__bytes_write.sum (a profiler is needed to
 # count them, so they cannot be measured inside this run), with the
 # schedule the autotuner picks for this scene; None for other workloads.
 # Keyed by FP32 (True) / FP64 (False).
-SOLVE_TRAFFIC_500 = {True: 439347456, False: 838375424}
+SOLVE_TRAFFIC_500 = {True: 434578688, False: 778064128}
 
 
 def roofline(sim, fp32, n=None):

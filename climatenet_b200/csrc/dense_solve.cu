@@ -30,7 +30,7 @@ __device__ __forceinline__ void dot16(double2 w, const double* b, double& s0, do
 // Bound by the launch and a few memory latencies for cloths of some hundred
 // vertices (30 x 30: 6.5 MB that stay in L2), by L2 bandwidth at the limit of
 // kDenseBytes.  The solve alone, events around it, sweeps in brackets: 30 x 30
-// 10 us (33), 53 x 53 25 us (45).
+// 12 us (33), 53 x 53 25 us (45).
 //
 // FP64 solves only.  An inverse kept in FP32 rounds each of its entries, and
 // nothing of that averages out over the rows as the sweeps' roundings do: v of

@@ -281,7 +281,7 @@ bool factorize(const Model& m, double dt, int leaf_size, Factor& f, std::string&
     // FP32 sweeps keep layers together: apart, their result was further
     // from the FP64 solve's by a fifth (two 256 x 256 layers, one step of 20
     // iterations, six inputs: 2.2e-6 to 2.4e-6
-    // relative against 2.0e-6), for all that a solve took 0.105 ms instead of 0.136
+    // relative against 2.0e-6), for all that a solve took 0.105 ms instead of 0.141
     std::vector<std::vector<int>> comps = gathered(components(m), std::max(8, leaf_size));
     if (fp32 && comps.size() > 1) comps = united(m, comps);
     for (std::vector<int>& ids : comps) {

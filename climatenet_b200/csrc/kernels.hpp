@@ -208,7 +208,7 @@ void launch_solve_prep(cudaStream_t st, int n, T* x, T* y, SweepSync sy);
 // (dense_solve.cu).  The inverse is kept where it takes at most kDenseBytes and
 // b fits the kernel's shared memory (two CTAs an SM).  Below the limit the product
 // reads L2-resident rows and beats the sweeps' chain of launches (30 x 30:
-// 6.5 MB, 10 us against 33; near the limit, 53 x 53: 25 us against 45); above
+// 6.5 MB, 12 us against 33; near the limit, 53 x 53: 25 us against 45); above
 // it the inverse grows with N^2 where the factor grows with N log N, and leaves L2.
 // Its construction (a third of N solves) replaces the schedule autotuner there:
 // creating a 30 x 30 cloth takes 13 ms (28 before).
