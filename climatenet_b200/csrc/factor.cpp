@@ -194,7 +194,8 @@ std::vector<std::vector<int>> united(const Model& m, const std::vector<std::vect
       const auto &a = box[by_ax[i]], &b = box[by_ax[j]];
       if (a[0] > b[3] || b[0] > a[3]) continue;
       // in the plane of the two widest extents layers cover each other; along the
-      // third they may lie apart
+      // third they may lie apart (0.05 of the side: far above the spacing of layers
+      // that touch, below that of cloths held apart; not measured in between)
       int over = 0;
       double gap = 0., side = 0.;
       for (int k = 0; k < 3; ++k) {
@@ -223,6 +224,7 @@ std::vector<std::vector<int>> united(const Model& m, const std::vector<std::vect
 // 24 N from two to three, N the scene's vertices.  FP64 solves: 9.4k vertices 49 us
 // at 3, 42 at 4 (5: 39, but the root's factorisation takes 100 ms instead of 24);
 // 15.6k 54 and 49; 22.5k 61 and 59; 40k 72 and 73; 250k 234 at 3, 230 at 2.
+// (N counts the scene, its components together.)
 // FP32 sweeps have three at every size: another factor rounds otherwise, and on small
 // cloths the roundings of the factor are most of what v differs by (24 x 24 on a
 // floor: twice as far from a run with three levels as two such runs are apart).
